@@ -32,6 +32,7 @@ UNITS = {
     "collide.cu": ["--fmad=false"],
     "mcc_fp32.cu": ["--use_fast_math"],
     "library.cu": [],
+    "pcg.cu": ["--fmad=false"],
     "pcg_static.cu": ["--fmad=false"],
     "unet_conv.cu": [],
     "unet.cu": [],

@@ -241,7 +241,9 @@ __device__ __forceinline__ double apply_M(const DMesh& m, const double* __restri
     return s;
 }
 
-// The PCG runs in the Chronopoulos-Gear form (one reduction point per
+// PCG of meshes beyond the persistent solve (pcg.cu, which states the sizes and
+// runs the same operations in the same order).  It runs in the
+// Chronopoulos-Gear form (one reduction point per
 // iteration): with u = D^-1 r, w = M u, s = M p,
 //   p = u + beta p,  s = w + beta s,  x += alpha p,  r -= alpha s,  u = D^-1 r
 //   w = M u,  gamma = r.u,  delta = w.u,  beta = gamma / gamma_old,

@@ -19,8 +19,28 @@ struct PcgState {
     double rz, rr, bb, pq, beta, lim, mean, of_residual, alpha;
     int done, iters, converged, k;
     unsigned int ticket;
-    unsigned int pad2[3];
+    // persistent solve (pcg.cu): wait counters, blocks gone, a wait ran out
+    unsigned int bar[3], exits;
+    int fail;
+    double rr0;   // r.r of the start guess
 };
+
+// Launch shape of the persistent solve (pcg.cu) for one problem size.
+struct PcgPlan {
+    int cells = 0;
+    int chunks = 0;     // kChunk cells each
+    int split = 1;      // blocks (one cluster) per chunk
+    int clusters = 0;
+    int smem = 0;
+    bool alone = false; // one block, at most 256 cells
+    bool fits = false;  // every block resident at once: the persistent solve runs
+};
+cudaError_t pcg_make_plan(int n, bool uniform, PcgPlan* plan);
+// The whole solve M x = b from the given x in one launch; u holds n doubles,
+// part 4 x pcg_blocks(n); st must be zero but for mean before the first solve
+// and after one that set st->fail.
+cudaError_t launch_pcg_solve(const DMesh& m, const PcgPlan& plan, const double* b, double* x, double* u, double* part,
+                             PcgState* st, double tol, int maxit, cudaStream_t s);
 
 // q * weight * 2^-kDepositBits per species (the FP32 form's fixed-point deposit).
 struct SpeciesValues {

@@ -313,7 +313,8 @@ struct picgpu_ctx {
     int64_t launches = 0;
     picgpu_step_stats acc{};
     cudaEvent_t timer[2] = {nullptr, nullptr};
-    cudaGraphExec_t pcg_graph = nullptr;
+    cudaGraphExec_t pcg_graph = nullptr;   // beyond the persistent solve's size
+    pgd::PcgPlan pcg_plan;
     double pcg_r0 = 0.0;  // ||b - A x0|| / ||b|| of the last solve's start guess
     std::unique_ptr<pgd::LearnedWarmStart> ws;  // learned warm start (cfg.learned.enabled)
     std::unique_ptr<pgd::MultigridPCG> mg;      // multigrid-preconditioned PCG (cfg.pcg_precond)
@@ -738,11 +739,12 @@ picgpu_status poisson(picgpu_ctx* c, picgpu_step_stats* stats, bool learned = fa
     const int maxit = c->cfg.pcg_max_iter > 0 ? c->cfg.pcg_max_iter : 10000;
     {
         PhaseScope ps(c, PICGPU_PHASE_POISSON);
-        // PCG iterations run as a CUDA graph of kGraphIters iterations
-        // (2 kernels each); iterations after convergence return at once, so
-        // the iteration count stays exact.  The host checks the done flag
-        // after each replay.
-        if (!c->pcg_graph && !c->mg) {
+        // Jacobi PCG: one persistent launch where every block fits the chip
+        // at once (pcg.cu); on larger meshes a CUDA graph of kGraphIters
+        // iterations (2 kernels each), where iterations after convergence
+        // return at once, so the iteration count stays exact, and the host
+        // checks the done flag after each replay.
+        if (!c->pcg_graph && !c->mg && !c->pcg_plan.fits) {
             cudaGraph_t g;
             CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
             for (int j = 0; j < kGraphIters; ++j)
@@ -776,6 +778,15 @@ picgpu_status poisson(picgpu_ctx* c, picgpu_step_stats* stats, bool learned = fa
             c->st_host->rr = rr;
             c->st_host->bb = bb;
             c->st_host->converged = conv ? 1 : 0;
+        } else if (c->pcg_plan.fits) {
+            CK(pgd::launch_pcg_solve(c->dm, c->pcg_plan, c->b, c->phi, c->z, c->part, c->st, tol, maxit, c->stream));
+            pgd::launch_of_residual(c->dm, c->b, c->phi, c->part, c->st, c->stream);
+            c->launches += 3;
+            CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
+            if (learned && c->ws) {
+                CK(cudaStreamSynchronize(c->stream));
+                CK(c->ws->after(c->dm, c->phi, c->st_host->iters, c->stream));
+            }
         } else {
             pgd::launch_pcg_init(c->dm, c->b, c->phi, c->r, c->z, c->q, c->part, c->st, tol, c->stream);
             c->launches += 2;
@@ -801,6 +812,13 @@ picgpu_status poisson(picgpu_ctx* c, picgpu_step_stats* stats, bool learned = fa
     CK(cudaStreamSynchronize(c->stream));
     (void)n;
     const pgd::PcgState& S = *c->st_host;
+    if (!c->mg && c->pcg_plan.fits) {
+        if (S.fail) {
+            CK(cudaMemset(c->st, 0, sizeof(pgd::PcgState)));
+            return bad(c, PICGPU_CUDA_ERROR, "Poisson PCG: a block of the solver kernel waited too long for the others");
+        }
+        c->pcg_r0 = S.bb > 0 ? std::sqrt(S.rr0 / S.bb) : 0.0;
+    }
     if (stats) {
         stats->pcg_iterations = S.iters;
         stats->pcg_iterations_total += S.iters;
@@ -1898,6 +1916,7 @@ static picgpu_status create_with_mesh(picgpu_ctx* c, const picgpu_config* cfg) {
         }
     }
     CK(cudaMemset(c->st, 0, sizeof(pgd::PcgState)));
+    CK(pgd::pcg_make_plan(int(nc), c->dm.lap_uniform != 0, &c->pcg_plan));
     CK(cudaMallocHost(&c->st_host, sizeof(pgd::PcgState)));
     CK(cudaMallocHost(&c->counters_host, sizeof(pgd::MoveCounters) * PICGPU_MAX_SPECIES));
     std::memset(c->st_host, 0, sizeof(pgd::PcgState));

@@ -1,6 +1,6 @@
 // pcg_static.cu -- allocation-free variant of the Poisson PCG.
 //
-// picgpu_solve_ldu_noalloc runs the same PCG kernels as picgpu_solve_poisson
+// picgpu_solve_ldu_noalloc runs the same PCG as picgpu_solve_poisson
 // (Jacobi preconditioner, fixed-order reductions) on a matrix and vectors the
 // caller already holds in device memory.  Its working vectors live in one
 // file-scope __device__ array instead of cudaMalloc'd buffers, so the call
@@ -88,8 +88,27 @@ extern "C" picgpu_status picgpu_solve_ldu_noalloc(int n_cells, const double* dia
     m.Moff = off;
     m.nbr = nbr;
     m.dinv = dinv;
-    pgd::launch_pcg_init(m, b, x, r, u, w, part, st, tol, s);
     pgd::PcgState h{};
+    pgd::PcgPlan plan;
+    if (pgd::pcg_make_plan(n_cells, false, &plan) != cudaSuccess) {
+        cudaGetLastError();
+        return PICGPU_CUDA_ERROR;
+    }
+    if (plan.fits) {
+        // the persistent solve (pcg.cu): every problem size on a GPU that
+        // holds kMaxBlocks blocks
+        if (pgd::launch_pcg_solve(m, plan, b, x, u, part, st, tol, max_iter, s) != cudaSuccess ||
+            cudaGetLastError() != cudaSuccess ||
+            cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+            cudaStreamSynchronize(s) != cudaSuccess || h.fail) {
+            cudaGetLastError();
+            return PICGPU_CUDA_ERROR;
+        }
+        if (iterations) *iterations = h.iters;
+        if (residual) *residual = h.bb > 0 ? std::sqrt(h.rr / h.bb) : 0.0;
+        return h.converged ? PICGPU_OK : PICGPU_PCG_NOT_CONVERGED;
+    }
+    pgd::launch_pcg_init(m, b, x, r, u, w, part, st, tol, s);
     // a launch error of the set-up kernels must not pass for convergence when
     // the start guess already meets the tolerance and no iteration runs
     if (cudaGetLastError() != cudaSuccess ||
