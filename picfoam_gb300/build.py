@@ -36,6 +36,7 @@ UNITS = {
     "pcg_static.cu": ["--fmad=false"],
     "unet_conv.cu": [],
     "unet.cu": [],
+    "unet_dw.cu": [],
     "learned.cu": [],
     "mg.cu": [],
     "init.cu": ["--fmad=false"],

@@ -2,7 +2,7 @@
 // (tcgen05: TMEM allocation, MMA issue, commit to an mbarrier, TMEM loads)
 // and the shared-memory operand descriptors of sm_100-family parts.
 //
-// Operand layout used throughout: K-major, no swizzle.  A tile of R rows x K
+// Operand layout of the convolution: K-major, no swizzle.  A tile of R rows x K
 // BF16 elements is stored as 8-row x 16-byte "core matrices"; core matrix
 // (row group g, K group j) sits at  base + j * kstride + g * 128  and holds
 // its 8 rows of 16 bytes contiguously.  kstride (the distance between core
@@ -40,6 +40,12 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
     return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(N >> 3) << 17) | (uint32_t(M >> 4) << 24);
 }
 
+// Both operands MN-major (bits 15, 16 = 1): a core matrix holds 8 K-rows of 16
+// bytes (8 M or N elements each); no swizzle: the leading-dimension byte
+// offset is the distance between core matrices adjacent in K, the
+// stride-dimension byte offset that between neighbours in M or N.
+constexpr uint32_t kMnMajorAB = (1u << 15) | (1u << 16);
+
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_addr(bar)), "r"(count) : "memory");
 }
@@ -60,6 +66,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "r"(smem_addr(bar)), "r"(parity)
         : "memory");
     return ok != 0;
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
 // Bounded wait for the completion of the phase with the given parity; false

@@ -21,7 +21,7 @@
 // packed from the FP32 master copy, accumulate in FP32.  Backward: the input
 // gradient of a tensor-core layer is the same tensor-core convolution with
 // the flipped, transposed weights (FP32 out); weight gradients accumulate in
-// FP32 on the CUDA cores.  Pooling is a 2x2x2 average, upsampling nearest.
+// FP32 on the tensor cores (unet_dw.cu).  Pooling is a 2x2x2 average, upsampling nearest.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -218,80 +218,6 @@ __global__ void pool_backward_kernel(ConvGrid g, int C, const float* __restrict_
     gfine[i] += 0.125f * gcoarse[vc * C + ch];
 }
 
-// Weight gradient dW[t][co][ci] += sum_v h[v][co] x[v + off_t][ci] on the CUDA
-// cores.  h is BF16 [V][COUT] (or FP32 [V] for COUT = 1), x is either the
-// concatenation of two BF16 sources (ConvSrc semantics) or FP32 [V][CIN].
-// Each thread owns P = COUT*CIN/256 (co, ci) pairs of one co row; a block
-// stages 128 voxels of h and of x's tap-shifted rows in shared memory.
-template <int CIN, int COUT, bool XF, bool HF>
-__global__ void __launch_bounds__(256) dw_kernel(ConvGrid g, const void* hp, ConvSrc s1, ConvSrc s2,
-                                                 const float* xf, float* __restrict__ dw) {
-    constexpr int kPairs = COUT * CIN;
-    constexpr int P = kPairs >= 256 ? kPairs / 256 : 1;
-    static_assert(kPairs < 256 || kPairs % 256 == 0, "pairs must tile the block");
-    static_assert(kPairs < 256 || CIN % P == 0, "a thread's pairs must share one co");
-    extern __shared__ float sm[];
-    float* sx = sm;                  // [128][CIN]
-    float* sh = sm + 128 * CIN;      // [128][COUT]
-    const int tid = threadIdx.x;
-    const long V = long(g.X) * g.Y * g.Z;
-    const long tiles = V / 128;
-    const int q0 = tid * P;
-    const bool active = q0 < kPairs;
-    const int co = active ? q0 / CIN : 0, ci0 = active ? q0 % CIN : 0;
-    for (int t = 0; t < 27; ++t) {
-        float acc[P];
-#pragma unroll
-        for (int k = 0; k < P; ++k) acc[k] = 0.f;
-        for (long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-            __syncthreads();
-            // stage h rows
-            for (int i = tid; i < 128 * COUT; i += 256) {
-                const long v = tile * 128 + i / COUT;
-                const int c = i % COUT;
-                sh[i] = HF ? static_cast<const float*>(hp)[v * COUT + c]
-                           : bf(static_cast<const __nv_bfloat16*>(hp)[v * COUT + c]);
-            }
-            // stage x rows shifted by tap t
-            for (int i = tid; i < 128 * CIN; i += 256) {
-                const int r = i / CIN, c = i % CIN;
-                const long v = tile * 128 + r;
-                const Coord cc = coord(v, g);
-                long nv;
-                float val = 0.f;
-                if (neighbour(cc, t, g, 1, &nv)) {
-                    if (XF) {
-                        val = xf[nv * CIN + c];
-                    } else {
-                        const Coord nc = coord(nv, g);
-                        if (c < s1.C) {
-                            const long idx = s1.up ? (long(nc.z >> 1) * (g.Y >> 1) + (nc.y >> 1)) * (g.X >> 1) + (nc.x >> 1)
-                                                   : nv;
-                            val = bf(s1.p[idx * s1.C + c]);
-                        } else {
-                            val = bf(s2.p[nv * s2.C + (c - s1.C)]);
-                        }
-                    }
-                }
-                sx[i] = val;
-            }
-            __syncthreads();
-            if (active) {
-                for (int r = 0; r < 128; ++r) {
-                    const float hv = sh[r * COUT + co];
-#pragma unroll
-                    for (int k = 0; k < P; ++k) acc[k] = fmaf(hv, sx[r * CIN + ci0 + k], acc[k]);
-                }
-            }
-        }
-        if (active) {
-#pragma unroll
-            for (int k = 0; k < P; ++k)
-                if (q0 + k < kPairs) atomicAdd(&dw[(size_t(t) * COUT + co) * CIN + ci0 + k], acc[k]);
-        }
-    }
-}
-
 // Adam (Kingma & Ba 2015) on one parameter array.
 __global__ void adam_kernel(long n, float* __restrict__ w, const float* __restrict__ gr, float* __restrict__ m,
                             float* __restrict__ v, float lr, float b1, float b2, float c1, float c2, float eps) {
@@ -359,16 +285,6 @@ cudaError_t zero(T* p, size_t n, cudaStream_t s) {
 }
 
 unsigned nblk(long n, int bs = 256) { return unsigned((n + bs - 1) / bs); }
-
-template <int CIN, int COUT, bool XF, bool HF>
-void launch_dw(const ConvGrid& g, const void* h, const ConvSrc& s1, const ConvSrc& s2, const float* xf, float* dw,
-               cudaStream_t s) {
-    const long tiles = long(g.X) * g.Y * g.Z / 128;
-    const int smem = 128 * (CIN + COUT) * int(sizeof(float));
-    auto k = dw_kernel<CIN, COUT, XF, HF>;
-    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    k<<<unsigned(std::min<long>(tiles, 1216)), 256, smem, s>>>(g, h, s1, s2, xf, dw);
-}
 
 }  // namespace
 
@@ -558,6 +474,15 @@ cudaError_t UNet::tc_dx(int l, const ConvGrid& g, float* gin, cudaStream_t s) {
     return launch_conv_tc(cout, cin, kEpiF32, g, {hb_, cout, 0}, none, wt_[l], gin, err_, s);
 }
 
+// Weight gradient of layer l from its output gradient (BF16 h, or FP32 h32
+// for the last layer); the first layer reads the FP32 network input.
+cudaError_t UNet::dw(int l, const ConvGrid& g, const __nv_bfloat16* h, ConvSrc s1, ConvSrc s2, const float* h32,
+                     cudaStream_t s) {
+    launches_ += 1;
+    return launch_dw_tc(kUNetLayers[l].cin, kUNetLayers[l].cout, g, h, h32, s1, s2, l == 0 ? in_ : nullptr,
+                        gw_ + off_[l], err_, s);
+}
+
 void UNet::mask(const float* gr, const __nv_bfloat16* a, long n, cudaStream_t s) {
     relu_mask_kernel<<<nblk(n), 256, 0, s>>>(n, gr, a, hb_);
     launches_ += 1;
@@ -566,58 +491,57 @@ void UNet::mask(const float* gr, const __nv_bfloat16* a, long n, cudaStream_t s)
 cudaError_t UNet::backward(cudaStream_t s) {
     const ConvSrc none{nullptr, 0, 0};
     const long V2 = V1_ / 8, V3 = V1_ / 64;
-    float* g = gw_;
     cudaError_t e;
     zero(gw_, nparam_, s);
     // out = co(a10)
-    launch_dw<16, 1, false, true>(g1_, gout_, {a_[10], 16, 0}, none, nullptr, g + off_[10], s);
+    if ((e = dw(10, g1_, nullptr, {a_[10], 16, 0}, none, gout_, s))) return e;
     conv_last_backward_kernel<<<nblk(V1_), 256, 0, s>>>(g1_, gout_, w_ + off_[10], gB_);
     // a10 = relu(d1b(a9))
     mask(gB_, a_[10], 16 * V1_, s);
-    launch_dw<16, 16, false, false>(g1_, hb_, {a_[9], 16, 0}, none, nullptr, g + off_[9], s);
+    if ((e = dw(9, g1_, hb_, {a_[9], 16, 0}, none, nullptr, s))) return e;
     if ((e = tc_dx(9, g1_, gB_, s))) return e;  // g_a9
     // a9 = relu(d1a([up(a8), a2]))
     mask(gB_, a_[9], 16 * V1_, s);
-    launch_dw<48, 16, false, false>(g1_, hb_, {a_[8], 32, 1}, {a_[2], 16, 0}, nullptr, g + off_[8], s);
+    if ((e = dw(8, g1_, hb_, {a_[8], 32, 1}, {a_[2], 16, 0}, nullptr, s))) return e;
     if ((e = tc_dx(8, g1_, gA_, s))) return e;  // g_cat [V1][48]
     zero(gskip1_, 16 * size_t(V1_), s);
     split_cat_kernel<<<nblk(V2), 256, 0, s>>>(g1_, 32, 16, gA_, gskip1_, gC_);  // g_a8 -> gC_ [V2][32]
     // a8 = relu(d2b(a7))
     mask(gC_, a_[8], 32 * V2, s);
-    launch_dw<32, 32, false, false>(g2_, hb_, {a_[7], 32, 0}, none, nullptr, g + off_[7], s);
+    if ((e = dw(7, g2_, hb_, {a_[7], 32, 0}, none, nullptr, s))) return e;
     if ((e = tc_dx(7, g2_, gB_, s))) return e;  // g_a7 [V2][32]
     // a7 = relu(d2a([up(a6), a4]))
     mask(gB_, a_[7], 32 * V2, s);
-    launch_dw<96, 32, false, false>(g2_, hb_, {a_[6], 64, 1}, {a_[4], 32, 0}, nullptr, g + off_[6], s);
+    if ((e = dw(6, g2_, hb_, {a_[6], 64, 1}, {a_[4], 32, 0}, nullptr, s))) return e;
     if ((e = tc_dx(6, g2_, gA_, s))) return e;  // g_cat [V2][96]
     zero(gskip2_, 32 * size_t(V2), s);
     split_cat_kernel<<<nblk(V3), 256, 0, s>>>(g2_, 64, 32, gA_, gskip2_, gC_);  // g_a6 -> gC_ [V3][64]
     // a6 = relu(c3b(a5))
     mask(gC_, a_[6], 64 * V3, s);
-    launch_dw<64, 64, false, false>(g3_, hb_, {a_[5], 64, 0}, none, nullptr, g + off_[5], s);
+    if ((e = dw(5, g3_, hb_, {a_[5], 64, 0}, none, nullptr, s))) return e;
     if ((e = tc_dx(5, g3_, gB_, s))) return e;  // g_a5 [V3][64]
     // a5 = relu(c3a(p2))
     mask(gB_, a_[5], 64 * V3, s);
-    launch_dw<32, 64, false, false>(g3_, hb_, {p2_, 32, 0}, none, nullptr, g + off_[4], s);
+    if ((e = dw(4, g3_, hb_, {p2_, 32, 0}, none, nullptr, s))) return e;
     if ((e = tc_dx(4, g3_, gC_, s))) return e;  // g_p2 [V3][32]
     pool_backward_kernel<<<nblk(32 * V2), 256, 0, s>>>(g2_, 32, gC_, gskip2_);  // g_a4 total
     // a4 = relu(c2b(a3))
     mask(gskip2_, a_[4], 32 * V2, s);
-    launch_dw<32, 32, false, false>(g2_, hb_, {a_[3], 32, 0}, none, nullptr, g + off_[3], s);
+    if ((e = dw(3, g2_, hb_, {a_[3], 32, 0}, none, nullptr, s))) return e;
     if ((e = tc_dx(3, g2_, gB_, s))) return e;  // g_a3 [V2][32]
     // a3 = relu(c2a(p1))
     mask(gB_, a_[3], 32 * V2, s);
-    launch_dw<16, 32, false, false>(g2_, hb_, {p1_, 16, 0}, none, nullptr, g + off_[2], s);
+    if ((e = dw(2, g2_, hb_, {p1_, 16, 0}, none, nullptr, s))) return e;
     if ((e = tc_dx(2, g2_, gC_, s))) return e;  // g_p1 [V2][16]
     pool_backward_kernel<<<nblk(16 * V1_), 256, 0, s>>>(g1_, 16, gC_, gskip1_);  // g_a2 total
     // a2 = relu(c1b(a1))
     mask(gskip1_, a_[2], 16 * V1_, s);
-    launch_dw<16, 16, false, false>(g1_, hb_, {a_[1], 16, 0}, none, nullptr, g + off_[1], s);
+    if ((e = dw(1, g1_, hb_, {a_[1], 16, 0}, none, nullptr, s))) return e;
     if ((e = tc_dx(1, g1_, gB_, s))) return e;  // g_a1
     // a1 = relu(c1a(in))
     mask(gB_, a_[1], 16 * V1_, s);
-    launch_dw<2, 16, true, false>(g1_, hb_, none, none, in_, g + off_[0], s);
-    launches_ += 30;
+    if ((e = dw(0, g1_, hb_, none, none, nullptr, s))) return e;
+    launches_ += 19;
     return cudaGetLastError();
 }
 

@@ -35,4 +35,13 @@ bool conv_tc_supported(int cin, int cout);
 cudaError_t launch_conv_tc(int cin, int cout, int epi, const ConvGrid& g, const ConvSrc& s1, const ConvSrc& s2,
                            const __nv_bfloat16* w, void* out, int* err, cudaStream_t st);
 
+// Weight gradient of such a convolution, added to dw (FP32 [27][cout][cin]):
+// dw[t][co][ci] += sum_v h[v][co] in[v + tap t][ci].  h is the BF16 output
+// gradient [V][cout], in the concatenation of s1 and s2; the first layer
+// (cin = 2, cout = 16) reads an FP32 input x32 [V][2] instead, the last
+// (cin = 16, cout = 1) an FP32 output gradient h32 [V].
+cudaError_t launch_dw_tc(int cin, int cout, const ConvGrid& g, const __nv_bfloat16* h, const float* h32,
+                         const ConvSrc& s1, const ConvSrc& s2, const float* x32, float* dw, int* err,
+                         cudaStream_t st);
+
 }  // namespace pgd

@@ -51,6 +51,8 @@ class UNet {
     void pack(cudaStream_t s);
     cudaError_t tc(int l, int epi, const ConvGrid& g, ConvSrc s1, ConvSrc s2, void* out, cudaStream_t s);
     cudaError_t tc_dx(int l, const ConvGrid& g, float* gin, cudaStream_t s);
+    cudaError_t dw(int l, const ConvGrid& g, const __nv_bfloat16* h, ConvSrc s1, ConvSrc s2, const float* h32,
+                   cudaStream_t s);
     void mask(const float* gr, const __nv_bfloat16* a, long n, cudaStream_t s);
 
     std::vector<void*> allocs_;
