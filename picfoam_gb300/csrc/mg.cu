@@ -37,18 +37,46 @@ namespace {
 constexpr int kInnerMax = 200;     // inner iterations per outer step
 constexpr int kOuterMax = 64;      // outer steps per solve
 constexpr double kEtaMin = 1e-4;   // deepest relative reduction asked of one FP32 inner solve
+// Factor of the linear prolongation on the correction scale: the scale
+// compensates for the stiffness of Galerkin operators of piecewise-constant
+// aggregation (1.6 was best with the piecewise-constant prolongation, 2.0 is
+// with the linear one).  Inner iterations to 1e-10, constant and linear
+// prolongation: 17 and 11 at 48^3, 18 and 10 at 64^3, 20 and 13 at 128^3.
+constexpr float kLinear = 1.25f;
+constexpr long kFuseVoxels = 40000;   // see vcycle()
+constexpr long kSmallVoxels = 600000; // see sum_planes()
+
+// Every kernel of a solve begins with after_previous(): its blocks may be set
+// up while the previous kernel still runs (programmatic dependent launch), and
+// wait there until it has finished and its writes are visible.  In a chain of
+// kernels of 2 to 3 us that hides part of a launch: 55.6 us per inner
+// iteration at 64^3 without it, 51.4 with it, 135 and 125 at 128^3.
+__device__ __forceinline__ void after_previous() {
+    asm volatile("griddepcontrol.launch_dependents;\ngriddepcontrol.wait;" ::: "memory");
+}
 
 // Level description passed by value to the FP32 kernels (32-bit indices:
 // a level holds fewer than 2^31 voxels).
 struct Lv {
     int X, Y, Z, cx, cy, cz;
     int V;
+    int zb;                 // planes per thread of the summing kernels
     int uniform;
     float coef[6];
     const float* __restrict__ diag;
     const float* __restrict__ inv;
     const float* __restrict__ off;
 };
+
+// What the prolongation from a level's aggregates needs: their grid, the
+// aggregation shifts, periodic axes and edge factors.
+struct Interp {
+    int n[3], s[3], cyc[3];
+    float edge[6];
+};
+
+constexpr int kZB = 8;
+int sum_planes(const MgLevel& L) { return L.V <= kSmallVoxels ? 1 : kZB; }
 
 Lv view(const MgLevel& L) {
     Lv v{};
@@ -59,6 +87,7 @@ Lv view(const MgLevel& L) {
     v.cy = L.cyc[1];
     v.cz = L.cyc[2];
     v.V = int(L.V);
+    v.zb = sum_planes(L);
     v.uniform = L.uniform;
     for (int f = 0; f < 6; ++f) v.coef[f] = L.coef[f];
     v.diag = L.diag;
@@ -95,13 +124,14 @@ Shape shape(int X, int Y, int Z) {
 
 Shape shape(const MgLevel& L) { return shape(L.n[0], L.n[1], L.n[2]); }
 
-// The level-0 kernels that end in a grid-wide sum give each thread kZB
-// z-planes, so that the last block combines kZB times fewer partials.
-constexpr int kZB = 4;
-
+// The level-0 kernels that end in a grid-wide sum give each thread up to kZB
+// z-planes: each block's ticket costs 1.8 ns at one address (128^3: 25 us per
+// sweep with a sum for 1 plane, 14.3 for 4, 13.3 for 8); on small grids one,
+// as the planes' latencies add up (48^3: 6.0 against 6.2 us, with p.q and q.z
+// 5.6 against 6.6).
 Shape shape_sum(const MgLevel& L) {
     Shape s = shape(L);
-    s.grid.z = (L.n[2] + kZB - 1) / kZB;
+    s.grid.z = (L.n[2] + sum_planes(L) - 1) / sum_planes(L);
     s.blocks = int(s.grid.x * s.grid.y * s.grid.z);
     return s;
 }
@@ -114,11 +144,11 @@ __device__ __forceinline__ bool coords(const Lv& L, int& i, int& j, int& k, int&
     return i < L.X && j < L.Y;
 }
 
-// Plane kz of the kZB planes of a shape_sum block.
+// Plane kz of the L.zb planes of a shape_sum block.
 __device__ __forceinline__ bool coords_sum(const Lv& L, int kz, int& i, int& j, int& k, int& v) {
     i = blockIdx.x * blockDim.x + threadIdx.x;
     j = blockIdx.y * blockDim.y + threadIdx.y;
-    k = blockIdx.z * kZB + kz;
+    k = blockIdx.z * L.zb + kz;
     v = i + L.X * (j + L.Y * k);
     return i < L.X && j < L.Y && k < L.Z;
 }
@@ -153,10 +183,35 @@ __device__ __forceinline__ float apply_A(const Lv& L, int i, int j, int k, int v
     return s;
 }
 
+// N sums over the nb partials of each (part + q nb) in one fixed order, by
+// 8 / N warps per sum; the results land in out[] (shared), valid after it.
+template <int N>
+__device__ __forceinline__ void final_sums(const double* part, int nb, double* out) {
+    __shared__ double wsum[8];
+    const int t = flat_tid(), w = t >> 5, lane = t & 31;
+    constexpr int W = 8 / N;
+    const double* p = part + (w / W) * nb;
+    double s = 0.0;
+#pragma unroll 4
+    for (int i = (w % W) * 32 + lane; i < nb; i += 32 * W) s = s + __ldcg(p + i);
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) s = s + __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) wsum[w] = s;
+    __syncthreads();
+    if (lane == 0 && w < N) {
+        double r = wsum[w * W];
+#pragma unroll
+        for (int k = 1; k < W; ++k) r = r + wsum[w * W + k];
+        out[w] = r;
+    }
+    __syncthreads();
+}
+
 // ------------------------------------------------------------ V-cycle ----
 // One sweep from a zero guess: y = omega D^-1 b.
 __global__ void __launch_bounds__(256) mg_smooth0_kernel(Lv L, const float* __restrict__ b, float* __restrict__ y,
                                                          float omega) {
+    after_previous();
     int i, j, k, v;
     if (!coords(L, i, j, k, v)) return;
     y[v] = (omega * L.inv[v]) * b[v];
@@ -167,6 +222,7 @@ __global__ void __launch_bounds__(256) mg_smooth0_kernel(Lv L, const float* __re
 template <bool Uniform>
 __global__ void __launch_bounds__(256) mg_smooth01_kernel(Lv L, const float* __restrict__ b, float* __restrict__ y,
                                                           float omega) {
+    after_previous();
     int i, j, k, v;
     if (!coords(L, i, j, k, v)) return;
     const float* __restrict__ inv = L.inv;
@@ -180,6 +236,7 @@ template <bool Uniform>
 __global__ void __launch_bounds__(256) mg_smooth_kernel(Lv L, const float* __restrict__ b,
                                                         const float* __restrict__ x, float* __restrict__ y,
                                                         float omega) {
+    after_previous();
     int i, j, k, v;
     if (!coords(L, i, j, k, v)) return;
     const float ax = apply_A<Uniform>(L, i, j, k, v, [&](int w) { return x[w]; });
@@ -193,8 +250,9 @@ __device__ __forceinline__ void finish_rz(float prod, float* wsf, double* ws, do
     const float bs = block_tree_f(prod, wsf);
     if (flat_tid() == 0) part[flat_bid()] = double(bs);
     if (arrive_last(&sc->ticket)) {
-        const double rz = final_sum(part, int(grid_blocks()), ws);
+        final_sums<1>(part, int(grid_blocks()), ws);
         if (flat_tid() == 0) {
+            const double rz = ws[0];
             const double rzo = sc->rz - sc->alpha * sc->qz;
             sc->beta = sc->k == 0 ? 0.0 : (rz - rzo) / sc->rz;
             sc->rz = rz;
@@ -207,11 +265,13 @@ template <bool Uniform>
 __global__ void __launch_bounds__(256) mg_smooth_dot_kernel(Lv L, const float* __restrict__ b,
                                                             const float* __restrict__ x, float* __restrict__ y,
                                                             float omega, double* part, MgScalars* sc) {
+    after_previous();
     __shared__ float wsf[256];
-    __shared__ double ws[256];
+    __shared__ double ws[2];
     float prod = 0.f;
 #pragma unroll
     for (int kz = 0; kz < kZB; ++kz) {
+        if (kz >= L.zb) break;
         int i, j, k, v;
         if (!coords_sum(L, kz, i, j, k, v)) continue;
         const float ax = apply_A<Uniform>(L, i, j, k, v, [&](int w) { return x[w]; });
@@ -226,11 +286,13 @@ __global__ void __launch_bounds__(256) mg_smooth_dot_kernel(Lv L, const float* _
 // r.z alone (no post sweeps, or a single-level hierarchy).
 __global__ void __launch_bounds__(256) mg_rz_kernel(Lv L, const float* __restrict__ r, const float* __restrict__ z,
                                                     double* part, MgScalars* sc) {
+    after_previous();
     __shared__ float wsf[256];
-    __shared__ double ws[256];
+    __shared__ double ws[2];
     float prod = 0.f;
 #pragma unroll
     for (int kz = 0; kz < kZB; ++kz) {
+        if (kz >= L.zb) break;
         int i, j, k, v;
         if (coords_sum(L, kz, i, j, k, v)) prod = fmaf(r[v], z[v], prod);
     }
@@ -238,92 +300,108 @@ __global__ void __launch_bounds__(256) mg_rz_kernel(Lv L, const float* __restric
 }
 
 // Coarse right-hand side: bc[I] = sum over the active children of I of
-// (b - A x), children in x-fastest order; sx, sy, sz are the aggregation
-// shifts (1: pairs, 0: none) of each axis.
+// (b - A x); sx, sy, sz are the aggregation shifts (1: pairs, 0: none) of each
+// axis.  A thread forms the two planes of a fine (i, j), and a warp holds 16 x
+// 2 of them, so the children along x and y meet in shuffles.  (One thread per
+// aggregate had an eighth of the threads in flight and eight stencils in a
+// row each; 2.7 us at 64^3 voxels now, 9.2 at 128^3.)
 template <bool Uniform>
 __global__ void __launch_bounds__(256) mg_restrict_kernel(Lv F, Lv Cl, int sx, int sy, int sz,
                                                           const float* __restrict__ b, const float* __restrict__ x,
                                                           float* __restrict__ bc) {
-    int ci, cj, ck, I;
-    if (!coords(Cl, ci, cj, ck, I)) return;
+    after_previous();
+    const int i = blockIdx.x * 16 + (threadIdx.x & 15), j = blockIdx.y * 16 + (threadIdx.x >> 4);
+    const int ck = blockIdx.z;
+    const bool in = i < F.X && j < F.Y;
     auto xv = [&](int w) { return x[w]; };
     float s = 0.f;
+    if (in) {
 #pragma unroll
-    for (int dz = 0; dz < 2; ++dz) {
-        const int k = (ck << sz) + dz;
-        if (dz > sz || k >= F.Z) continue;
-#pragma unroll
-        for (int dy = 0; dy < 2; ++dy) {
-            const int j = (cj << sy) + dy;
-            if (dy > sy || j >= F.Y) continue;
-#pragma unroll
-            for (int dx = 0; dx < 2; ++dx) {
-                const int i = (ci << sx) + dx;
-                if (dx > sx || i >= F.X) continue;
-                const int v = i + F.X * (j + F.Y * k);
-                if (F.inv[v] != 0.f) s += b[v] - apply_A<Uniform>(F, i, j, k, v, xv);
-            }
+        for (int dz = 0; dz < 2; ++dz) {
+            const int k = (ck << sz) + dz;
+            if (dz > sz || k >= F.Z) continue;
+            const int v = i + F.X * (j + F.Y * k);
+            const float r = b[v] - apply_A<Uniform>(F, i, j, k, v, xv);
+            if (F.inv[v] != 0.f) s += r;
         }
     }
-    bc[I] = s;
+    // threads outside the grid hold zero
+    if (sx) s += __shfl_down_sync(0xffffffffu, s, 1);
+    if (sy) s += __shfl_down_sync(0xffffffffu, s, 16);
+    if (in && !(sx && (i & 1)) && !(sy && (j & 1))) bc[(i >> sx) + Cl.X * ((j >> sy) + Cl.Y * ck)] = s;
 }
 
-// x += scale * xc[parent] on the active voxels.
-__global__ void __launch_bounds__(256) mg_prolong_kernel(Lv F, int CX, int CY, int sx, int sy, int sz,
-                                                         const float* __restrict__ xc, float* __restrict__ x,
-                                                         float scale) {
+// The coarse correction at fine voxel (i, j, k), interpolated linearly between
+// the aggregate centres (weights 3/4 and 1/4 per paired axis).  Beyond a
+// non-periodic edge the coarse value is edge x its mirror image: -1 where the
+// potential is given there (the correction is zero on that face), +1 where
+// its gradient is.
+__device__ __forceinline__ float coarse_at(const Interp& P, int i, int j, int k, const float* __restrict__ xc) {
+    const int ci = i >> P.s[0], cj = j >> P.s[1], ck = k >> P.s[2];
+    // the neighbour aggregate on the child's side, per axis
+    int ni = ci + ((i & 1) ? 1 : -1), nj = cj + ((j & 1) ? 1 : -1), nk = ck + ((k & 1) ? 1 : -1);
+    float wi = 0.25f, wj = 0.25f, wk = 0.25f, ai = 0.75f, aj = 0.75f, ak = 0.75f;
+    if (!P.s[0]) { ni = ci; wi = 0.f; ai = 1.f; }
+    else if (ni < 0) { if (P.cyc[0]) ni = P.n[0] - 1; else { ni = ci; wi *= P.edge[0]; } }
+    else if (ni >= P.n[0]) { if (P.cyc[0]) ni = 0; else { ni = ci; wi *= P.edge[1]; } }
+    if (!P.s[1]) { nj = cj; wj = 0.f; aj = 1.f; }
+    else if (nj < 0) { if (P.cyc[1]) nj = P.n[1] - 1; else { nj = cj; wj *= P.edge[2]; } }
+    else if (nj >= P.n[1]) { if (P.cyc[1]) nj = 0; else { nj = cj; wj *= P.edge[3]; } }
+    if (!P.s[2]) { nk = ck; wk = 0.f; ak = 1.f; }
+    else if (nk < 0) { if (P.cyc[2]) nk = P.n[2] - 1; else { nk = ck; wk *= P.edge[4]; } }
+    else if (nk >= P.n[2]) { if (P.cyc[2]) nk = 0; else { nk = ck; wk *= P.edge[5]; } }
+    const int X = P.n[0], XY = P.n[0] * P.n[1];
+    const float* r0 = xc + XY * ck;
+    const float* r1 = xc + XY * nk;
+    const float p00 = fmaf(ai, r0[ci + X * cj], wi * r0[ni + X * cj]);
+    const float p01 = fmaf(ai, r0[ci + X * nj], wi * r0[ni + X * nj]);
+    const float p10 = fmaf(ai, r1[ci + X * cj], wi * r1[ni + X * cj]);
+    const float p11 = fmaf(ai, r1[ci + X * nj], wi * r1[ni + X * nj]);
+    return fmaf(ak, fmaf(aj, p00, wj * p01), wk * fmaf(aj, p10, wj * p11));
+}
+
+// x += scale * (coarse correction) on the active voxels.
+__global__ void __launch_bounds__(256) mg_prolong_kernel(Lv F, Interp P, const float* __restrict__ xc,
+                                                         float* __restrict__ x, float scale) {
+    after_previous();
     int i, j, k, v;
     if (!coords(F, i, j, k, v)) return;
     if (F.inv[v] == 0.f) return;
-    const int I = (i >> sx) + CX * ((j >> sy) + CY * (k >> sz));
-    x[v] = fmaf(scale, xc[I], x[v]);
+    x[v] = fmaf(scale, coarse_at(P, i, j, k, xc), x[v]);
 }
 
-// The prolongation fused into the first post sweep: x' = x + scale xc[parent]
-// on the active voxels (zero on holes), formed at the seven stencil points
-// from their own (i, j, k), then y = x' + omega D^-1 (b - A x').
+// The prolongation inside the first post sweep: x' = x + scale * (coarse
+// correction) on the active voxels (zero on holes) is formed at the seven
+// stencil points, y = x' + omega D^-1 (b - A x').
 template <bool Uniform>
-__global__ void __launch_bounds__(256) mg_prolong_smooth_kernel(Lv L, int CX, int CY, int sx, int sy, int sz,
-                                                                const float* __restrict__ xc,
+__global__ void __launch_bounds__(256) mg_prolong_smooth_kernel(Lv L, Interp P, const float* __restrict__ xc,
                                                                 const float* __restrict__ b,
                                                                 const float* __restrict__ x, float* __restrict__ y,
                                                                 float scale, float omega) {
+    after_previous();
     int i, j, k, v;
     if (!coords(L, i, j, k, v)) return;
-    const int X = L.X, XY = L.X * L.Y;
-    auto xp = [&](int w, int wi, int wj, int wk) {
+    auto at = [&](int w, int wi, int wj, int wk) {
         if (L.inv[w] == 0.f) return 0.f;
-        return fmaf(scale, xc[(wi >> sx) + CX * ((wj >> sy) + CY * (wk >> sz))], x[w]);
+        return fmaf(scale, coarse_at(P, wi, wj, wk, xc), x[w]);
     };
-    // neighbours: index and coordinates, with the periodic wrap; across a
-    // non-periodic edge the point is v itself with a zero coefficient
-    int ni[6], nj[6], nk[6], nb[6];
-    bool ok[6];
-    ok[0] = i > 0 || L.cx;
-    ni[0] = i > 0 ? i - 1 : (L.cx ? L.X - 1 : i);
-    ok[1] = i < L.X - 1 || L.cx;
-    ni[1] = i < L.X - 1 ? i + 1 : (L.cx ? 0 : i);
-    nj[0] = nj[1] = j;
-    nk[0] = nk[1] = k;
-    ok[2] = j > 0 || L.cy;
-    nj[2] = j > 0 ? j - 1 : (L.cy ? L.Y - 1 : j);
-    ok[3] = j < L.Y - 1 || L.cy;
-    nj[3] = j < L.Y - 1 ? j + 1 : (L.cy ? 0 : j);
-    ni[2] = ni[3] = i;
-    nk[2] = nk[3] = k;
-    ok[4] = k > 0 || L.cz;
-    nk[4] = k > 0 ? k - 1 : (L.cz ? L.Z - 1 : k);
-    ok[5] = k < L.Z - 1 || L.cz;
-    nk[5] = k < L.Z - 1 ? k + 1 : (L.cz ? 0 : k);
-    ni[4] = ni[5] = i;
-    nj[4] = nj[5] = j;
-    for (int f = 0; f < 6; ++f) nb[f] = ni[f] + X * nj[f] + XY * nk[f];
-    const float xv = xp(v, i, j, k);
+    // neighbours with the periodic wrap; across a non-periodic edge the point
+    // is v itself with a zero coefficient
+    const int im = i > 0 ? i - 1 : (L.cx ? L.X - 1 : i), ip = i < L.X - 1 ? i + 1 : (L.cx ? 0 : i);
+    const int jm = j > 0 ? j - 1 : (L.cy ? L.Y - 1 : j), jp = j < L.Y - 1 ? j + 1 : (L.cy ? 0 : j);
+    const int km = k > 0 ? k - 1 : (L.cz ? L.Z - 1 : k), kp = k < L.Z - 1 ? k + 1 : (L.cz ? 0 : k);
+    const bool ok[6] = {i > 0 || L.cx, i < L.X - 1 || L.cx, j > 0 || L.cy,
+                        j < L.Y - 1 || L.cy, k > 0 || L.cz, k < L.Z - 1 || L.cz};
+    const int X = L.X, XY = L.X * L.Y;
+    const float u[6] = {at(v + im - i, im, j, k),        at(v + ip - i, ip, j, k),
+                        at(v + X * (jm - j), i, jm, k),  at(v + X * (jp - j), i, jp, k),
+                        at(v + XY * (km - k), i, j, km), at(v + XY * (kp - k), i, j, kp)};
+    const float xv = at(v, i, j, k);
     float s = L.diag[v] * xv;
 #pragma unroll
     for (int f = 0; f < 6; ++f) {
         const float a = Uniform ? (ok[f] ? L.coef[f] : 0.f) : L.off[f * L.V + v];
-        s = fmaf(a, xp(nb[f], ni[f], nj[f], nk[f]), s);
+        s = fmaf(a, u[f], s);
     }
     y[v] = fmaf(omega * L.inv[v], b[v] - s, xv);
 }
@@ -332,6 +410,7 @@ __global__ void __launch_bounds__(256) mg_prolong_smooth_kernel(Lv L, int CX, in
 // lane l adds k = l, l + 32, ... then an xor-tree.
 __global__ void __launch_bounds__(256) mg_coarse_kernel(const float* __restrict__ inv, const int* __restrict__ idx,
                                                         int nc, const float* __restrict__ b, float* __restrict__ x) {
+    after_previous();
     const int row = int((long(blockIdx.x) * 256 + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (row >= nc) return;
@@ -352,6 +431,7 @@ __global__ void __launch_bounds__(256) mg_coarse_kernel(const float* __restrict_
 template <bool Uniform>
 __global__ void __launch_bounds__(256) mg_spmv_kernel(Lv L, const float* __restrict__ z, float* __restrict__ pb,
                                                       float* __restrict__ q, double* part, MgScalars* sc) {
+    after_previous();
     __shared__ float wsf[256];
     __shared__ double ws[256];
     const int it = sc->k;
@@ -362,6 +442,7 @@ __global__ void __launch_bounds__(256) mg_spmv_kernel(Lv L, const float* __restr
     float spq = 0.f, sqz = 0.f;
 #pragma unroll
     for (int kz = 0; kz < kZB; ++kz) {
+        if (kz >= L.zb) break;
         int i, j, k, v;
         if (!coords_sum(L, kz, i, j, k, v)) continue;
         const float pc = pv(v);
@@ -380,9 +461,9 @@ __global__ void __launch_bounds__(256) mg_spmv_kernel(Lv L, const float* __restr
         part[nb + flat_bid()] = double(b1);
     }
     if (arrive_last(&sc->ticket)) {
-        const double pq = final_sum(part, nb, ws);
-        const double qz = final_sum(part + nb, nb, ws);
+        final_sums<2>(part, nb, ws);
         if (flat_tid() == 0) {
+            const double pq = ws[0], qz = ws[1];
             sc->qz = qz;
             if (pq > 0.0 && sc->rz > 0.0) {
                 sc->alpha = sc->rz / pq;
@@ -400,6 +481,7 @@ __global__ void __launch_bounds__(256) mg_axpy_kernel(Lv L, float* __restrict__ 
                                                       const float* __restrict__ pb, const float* __restrict__ q,
                                                       double* part, MgScalars* sc, unsigned int* guard,
                                                       int maxit, cudaGraphConditionalHandle inner, int graph) {
+    after_previous();
     __shared__ float wsf[256];
     __shared__ double ws[256];
     const float alpha = float(sc->alpha);
@@ -407,6 +489,7 @@ __global__ void __launch_bounds__(256) mg_axpy_kernel(Lv L, float* __restrict__ 
     float srr = 0.f;
 #pragma unroll
     for (int kz = 0; kz < kZB; ++kz) {
+        if (kz >= L.zb) break;
         int i, j, k, v;
         if (!coords_sum(L, kz, i, j, k, v)) continue;
         d[v] = fmaf(alpha, p[v], d[v]);
@@ -417,8 +500,9 @@ __global__ void __launch_bounds__(256) mg_axpy_kernel(Lv L, float* __restrict__ 
     const float bs = block_tree_f(srr, wsf);
     if (flat_tid() == 0) part[flat_bid()] = double(bs);
     if (arrive_last(&sc->ticket)) {
-        const double rr = final_sum(part, int(grid_blocks()), ws);
+        final_sums<1>(part, int(grid_blocks()), ws);
         if (flat_tid() == 0) {
+            const double rr = ws[0];
             const int kk = sc->k + 1;
             const int total = sc->total + 1;
             const unsigned int g = *guard + 1u;
@@ -457,6 +541,7 @@ __global__ void __launch_bounds__(256) mg_residual_kernel(DMesh m, const double*
                                                           double* part, MgScalars* sc, int first, double tol,
                                                           int maxit, unsigned int* guard,
                                                           cudaGraphConditionalHandle outer, int graph) {
+    after_previous();
     __shared__ double ws[256];
     const int n = m.n_cells;
     const int nb = gridDim.x;
@@ -520,6 +605,7 @@ __global__ void __launch_bounds__(256) mg_convert_kernel(int n, const int* __res
                                                          const double* __restrict__ r, float* __restrict__ r32,
                                                          float* __restrict__ d, double* part, MgScalars* sc,
                                                          int maxit, cudaGraphConditionalHandle inner, int graph) {
+    after_previous();
     __shared__ float wsf[256];
     __shared__ double ws[256];
     const double scale = sc->scale;
@@ -556,9 +642,24 @@ __global__ void __launch_bounds__(256) mg_convert_kernel(int n, const int* __res
 __global__ void __launch_bounds__(256) mg_update_kernel(int n, const int* __restrict__ vox,
                                                         const float* __restrict__ d, double* __restrict__ x,
                                                         const MgScalars* sc) {
+    after_previous();
     const long i = long(blockIdx.x) * 256 + threadIdx.x;
     if (i >= n) return;
     x[i] = fma(double(d[vox[i]]), sc->inv_scale, x[i]);
+}
+
+template <class... P, class... A>
+void launch(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
 inline int nblk(long n, int bs) { return int((n + bs - 1) / bs); }
@@ -830,6 +931,14 @@ bool MultigridPCG::init(const pg::HexMesh& m, const std::vector<double>& Mdiag, 
         vox[c] = int(vidx(hl[0], m.cell_ijk[3 * size_t(c)], m.cell_ijk[3 * size_t(c) + 1],
                           m.cell_ijk[3 * size_t(c) + 2]));
     const long V0 = hl[0].V;
+    // the correction vanishes on a side whose potential is given (an RLC
+    // cathode's too, nearly) and is flat across one whose gradient is
+    for (int f = 0; f < 6; ++f) {
+        const auto& p = m.patches[f].p;
+        const int rule = pg::face_rule(p.kind, p.phi_bc);
+        const bool given = p.kind != PICGPU_PATCH_EMPTY && (rule == pg::kRuleFixed || rule == pg::kRuleRlc);
+        edge_[f] = given ? -1.f : 1.f;
+    }
     // block partials: the widest reduction launch (cells, or the level-0 grid)
     const long nbmax = std::max<long>(pcg_blocks(m.n_cells), shape(lv_[0]).blocks);
     part_cap_ = 2 * nbmax + 8;
@@ -875,70 +984,76 @@ int MultigridPCG::vcycle(int l, cudaStream_t s) {
     const Shape sh = shape(L);
     const float om = float(set_.omega);
     if (l == int(lv_.size()) - 1) {
-        mg_coarse_kernel<<<nblk(32L * nc_, 256), 256, 0, s>>>(cinv_, cidx_, nc_, L.b, L.x);
+        launch(mg_coarse_kernel, nblk(32L * nc_, 256), 256, s, cinv_, cidx_, nc_, L.b, L.x);
         if (l > 0) return 1;
         const Shape ss = shape_sum(L);
-        mg_rz_kernel<<<ss.grid, ss.block, 0, s>>>(v, L.b, L.x, part_, sc_);
+        launch(mg_rz_kernel, ss.grid, ss.block, s, v, L.b, L.x, part_, sc_);
         return 2;
     }
     int launched = 0;
     float* cur = L.x;
     float* oth = L.t;
     if (set_.pre == 1) {
-        mg_smooth0_kernel<<<sh.grid, sh.block, 0, s>>>(v, L.b, cur, om);
+        launch(mg_smooth0_kernel, sh.grid, sh.block, s, v, L.b, cur, om);
     } else {
-        if (L.uniform) mg_smooth01_kernel<true><<<sh.grid, sh.block, 0, s>>>(v, L.b, cur, om);
-        else mg_smooth01_kernel<false><<<sh.grid, sh.block, 0, s>>>(v, L.b, cur, om);
+        if (L.uniform) launch(mg_smooth01_kernel<true>, sh.grid, sh.block, s, v, L.b, cur, om);
+        else launch(mg_smooth01_kernel<false>, sh.grid, sh.block, s, v, L.b, cur, om);
     }
     ++launched;
     for (int it = 2; it < set_.pre; ++it) {
-        if (L.uniform) mg_smooth_kernel<true><<<sh.grid, sh.block, 0, s>>>(v, L.b, cur, oth, om);
-        else mg_smooth_kernel<false><<<sh.grid, sh.block, 0, s>>>(v, L.b, cur, oth, om);
+        if (L.uniform) launch(mg_smooth_kernel<true>, sh.grid, sh.block, s, v, L.b, cur, oth, om);
+        else launch(mg_smooth_kernel<false>, sh.grid, sh.block, s, v, L.b, cur, oth, om);
         std::swap(cur, oth);
         ++launched;
     }
     const MgLevel& C = lv_[l + 1];
     const Lv cv = view(C);
-    const Shape cs = shape(C);
+    const dim3 rg((L.n[0] + 15) / 16, (L.n[1] + 15) / 16, C.n[2]);
     const int sx = L.fac[0] - 1, sy = L.fac[1] - 1, sz = L.fac[2] - 1;
     if (L.uniform)
-        mg_restrict_kernel<true><<<cs.grid, cs.block, 0, s>>>(v, cv, sx, sy, sz, L.b, cur, C.b);
+        launch(mg_restrict_kernel<true>, rg, 256, s, v, cv, sx, sy, sz, L.b, cur, C.b);
     else
-        mg_restrict_kernel<false><<<cs.grid, cs.block, 0, s>>>(v, cv, sx, sy, sz, L.b, cur, C.b);
+        launch(mg_restrict_kernel<false>, rg, 256, s, v, cv, sx, sy, sz, L.b, cur, C.b);
     ++launched;
     launched += vcycle(l + 1, s);
-    const bool fuse = set_.post >= 1 && !(l == 0 && set_.post == 1);
+    Interp P{};
+    for (int a = 0; a < 3; ++a) {
+        P.n[a] = C.n[a];
+        P.s[a] = L.fac[a] - 1;
+        P.cyc[a] = C.cyc[a];
+    }
+    for (int f = 0; f < 6; ++f) P.edge[f] = edge_[f];
+    // on small levels a launch costs more than forming the correction seven
+    // times in the first post sweep (above 40,000 voxels the fused form is
+    // 4 to 7 us per iteration slower)
+    const bool fuse = L.V <= kFuseVoxels && set_.post >= 1 && !(l == 0 && set_.post == 1);
+    const float scale = kLinear * float(set_.scale);
     if (fuse) {
-        // the prolongation inside the first post sweep
         if (L.uniform)
-            mg_prolong_smooth_kernel<true><<<sh.grid, sh.block, 0, s>>>(v, C.n[0], C.n[1], sx, sy, sz, result(l + 1),
-                                                                        L.b, cur, oth, float(set_.scale), om);
+            launch(mg_prolong_smooth_kernel<true>, sh.grid, sh.block, s, v, P, result(l + 1), L.b, cur, oth, scale, om);
         else
-            mg_prolong_smooth_kernel<false><<<sh.grid, sh.block, 0, s>>>(v, C.n[0], C.n[1], sx, sy, sz,
-                                                                         result(l + 1), L.b, cur, oth,
-                                                                         float(set_.scale), om);
+            launch(mg_prolong_smooth_kernel<false>, sh.grid, sh.block, s, v, P, result(l + 1), L.b, cur, oth, scale, om);
         std::swap(cur, oth);
     } else {
-        mg_prolong_kernel<<<sh.grid, sh.block, 0, s>>>(v, C.n[0], C.n[1], sx, sy, sz, result(l + 1), cur,
-                                                      float(set_.scale));
+        launch(mg_prolong_kernel, sh.grid, sh.block, s, v, P, result(l + 1), cur, scale);
     }
     ++launched;
     for (int it = fuse ? 1 : 0; it < set_.post; ++it) {
         const bool last0 = l == 0 && it == set_.post - 1;
         if (last0) {
             const Shape ss = shape_sum(L);
-            if (L.uniform) mg_smooth_dot_kernel<true><<<ss.grid, ss.block, 0, s>>>(v, L.b, cur, oth, om, part_, sc_);
-            else mg_smooth_dot_kernel<false><<<ss.grid, ss.block, 0, s>>>(v, L.b, cur, oth, om, part_, sc_);
+            if (L.uniform) launch(mg_smooth_dot_kernel<true>, ss.grid, ss.block, s, v, L.b, cur, oth, om, part_, sc_);
+            else launch(mg_smooth_dot_kernel<false>, ss.grid, ss.block, s, v, L.b, cur, oth, om, part_, sc_);
         } else {
-            if (L.uniform) mg_smooth_kernel<true><<<sh.grid, sh.block, 0, s>>>(v, L.b, cur, oth, om);
-            else mg_smooth_kernel<false><<<sh.grid, sh.block, 0, s>>>(v, L.b, cur, oth, om);
+            if (L.uniform) launch(mg_smooth_kernel<true>, sh.grid, sh.block, s, v, L.b, cur, oth, om);
+            else launch(mg_smooth_kernel<false>, sh.grid, sh.block, s, v, L.b, cur, oth, om);
         }
         std::swap(cur, oth);
         ++launched;
     }
     if (l == 0 && set_.post == 0) {
         const Shape ss = shape_sum(L);
-        mg_rz_kernel<<<ss.grid, ss.block, 0, s>>>(v, L.b, cur, part_, sc_);
+        launch(mg_rz_kernel, ss.grid, ss.block, s, v, L.b, cur, part_, sc_);
         ++launched;
     }
     return launched;
@@ -952,9 +1067,9 @@ int MultigridPCG::inner_iteration(cudaStream_t s, int maxit, cudaGraphConditiona
     const Shape sh = shape_sum(L0);
     int launched = vcycle(0, s);
     float* z = result(0);
-    if (L0.uniform) mg_spmv_kernel<true><<<sh.grid, sh.block, 0, s>>>(v0, z, p_, q_, part_, sc_);
-    else mg_spmv_kernel<false><<<sh.grid, sh.block, 0, s>>>(v0, z, p_, q_, part_, sc_);
-    mg_axpy_kernel<<<sh.grid, sh.block, 0, s>>>(v0, d_, L0.b, p_, q_, part_, sc_, guard_, maxit, h_inner, graph);
+    if (L0.uniform) launch(mg_spmv_kernel<true>, sh.grid, sh.block, s, v0, z, p_, q_, part_, sc_);
+    else launch(mg_spmv_kernel<false>, sh.grid, sh.block, s, v0, z, p_, q_, part_, sc_);
+    launch(mg_axpy_kernel, sh.grid, sh.block, s, v0, d_, L0.b, p_, q_, part_, sc_, guard_, maxit, h_inner, graph);
     return launched + 2;
 }
 
@@ -962,10 +1077,10 @@ void MultigridPCG::residual(const DMesh& dm, const double* b, double* x, int fir
                             cudaStream_t s, cudaGraphConditionalHandle h_outer, int graph) {
     const int nbc = pcg_blocks(n_cells_);
     if (dm.lap_uniform)
-        mg_residual_kernel<true><<<nbc, 256, 0, s>>>(dm, b, x, r64_, part_, sc_, first, tol, maxit, guard_, h_outer,
+        launch(mg_residual_kernel<true>, nbc, 256, s, dm, b, x, r64_, part_, sc_, first, tol, maxit, guard_, h_outer,
                                                       graph);
     else
-        mg_residual_kernel<false><<<nbc, 256, 0, s>>>(dm, b, x, r64_, part_, sc_, first, tol, maxit, guard_, h_outer,
+        launch(mg_residual_kernel<false>, nbc, 256, s, dm, b, x, r64_, part_, sc_, first, tol, maxit, guard_, h_outer,
                                                        graph);
 }
 
@@ -1028,7 +1143,7 @@ cudaError_t MultigridPCG::build_graph(const DMesh& dm, const double* b, double* 
     if ((e = add_while(main, tail, h_outer, &w_outer, &body_outer))) return fail(e);
     if ((e = cudaGraphConditionalHandleCreate(&h_inner, body_outer, 0, cudaGraphCondAssignDefault))) return fail(e);
     e = capture(body_outer, {}, [&] {
-        mg_convert_kernel<<<nbc, 256, 0, s>>>(n, vox_, r64_, lv_[0].b, d_, part_, sc_, maxit, h_inner, 1);
+        launch(mg_convert_kernel, nbc, 256, s, n, vox_, r64_, lv_[0].b, d_, part_, sc_, maxit, h_inner, 1);
     }, &tail);
     if (e) return fail(e);
     if ((e = add_while(body_outer, tail, h_inner, &w_inner, &body_inner))) return fail(e);
@@ -1036,7 +1151,7 @@ cudaError_t MultigridPCG::build_graph(const DMesh& dm, const double* b, double* 
     e = capture(body_inner, {}, [&] { inner = inner_iteration(s, maxit, h_inner, 1); }, nullptr);
     if (e) return fail(e);
     e = capture(body_outer, {w_inner}, [&] {
-        mg_update_kernel<<<nblk(n, 256), 256, 0, s>>>(n, vox_, d_, x, sc_);
+        launch(mg_update_kernel, nblk(n, 256), 256, s, n, vox_, d_, x, sc_);
         residual(dm, b, x, 0, tol, maxit, s, h_outer, 1);
     }, nullptr);
     if (e) return fail(e);
@@ -1068,14 +1183,14 @@ cudaError_t MultigridPCG::solve_eager(const DMesh& dm, const double* b, double* 
     launches += 1;
     if ((e = read())) return e;
     while (!sc_host_->done) {
-        mg_convert_kernel<<<nbc, 256, 0, s>>>(n, vox_, r64_, lv_[0].b, d_, part_, sc_, maxit, 0, 0);
+        launch(mg_convert_kernel, nbc, 256, s, n, vox_, r64_, lv_[0].b, d_, part_, sc_, maxit, 0, 0);
         launches += 1;
         if ((e = read())) return e;
         while (!sc_host_->idone) {
             launches += inner_iteration(s, maxit, 0, 0);
             if ((e = read())) return e;
         }
-        mg_update_kernel<<<nblk(n, 256), 256, 0, s>>>(n, vox_, d_, x, sc_);
+        launch(mg_update_kernel, nblk(n, 256), 256, s, n, vox_, d_, x, sc_);
         residual(dm, b, x, 0, tol, maxit, s, 0, 0);
         launches += 2;
         if ((e = read())) return e;

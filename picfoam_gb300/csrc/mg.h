@@ -5,7 +5,8 @@
 // full voxel grid (voxels of removed box cells are holes: no equation, value
 // zero), so every level addresses its neighbours by index arithmetic.  Level
 // l + 1 aggregates 2x2x2 voxels of level l (ceil(n/2) aggregates per axis);
-// its operator is the Galerkin product P^T A P with piecewise-constant P:
+// its operator is the Galerkin product P^T A P with piecewise-constant P (the
+// correction itself is prolonged linearly):
 // face couplings summed across aggregate faces, diagonals and internal
 // couplings summed into the diagonal.  One preconditioner application is a
 // V-cycle: weighted-Jacobi sweeps before and after the scaled coarse
@@ -93,6 +94,7 @@ class MultigridPCG {
     float* cinv_ = nullptr;        // dense inverse, nc_ x nc_
     int* vox_ = nullptr;           // voxel of each cell
     int n_cells_ = 0;
+    float edge_[6] = {};           // of the sides: coarse correction beyond the edge / its mirror image
     double* r64_ = nullptr;        // FP64 residual over the cells
     float *d_ = nullptr, *p_ = nullptr, *q_ = nullptr;  // inner vectors on the level-0 grid
     double* part_ = nullptr;
