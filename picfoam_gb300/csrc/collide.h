@@ -48,6 +48,7 @@ struct MccParams {
     unsigned long long* counts;
     long stage_cap;       // staging slots; a cell whose candidates do not fit drops its secondaries
     int* overflow;        // raised when that happens
+    int* flags;           // per staging slot: 1 electron, 2 ion to append
     unsigned long long* iz_cell;  // optional ionisations per cell
     const unsigned* step_dev;     // optional: the step index read on the device (graph replays)
 };
@@ -100,7 +101,8 @@ struct CollideState {
     int* cell_start = nullptr;    // per species: n_cells + 1 offsets into idx
     int* cell_count = nullptr;
     int* cell_cursor = nullptr;
-    int* scan_tmp = nullptr;
+    int* scan_tmp = nullptr;      // state of the prefix sums over the cells
+    // kCollideCounts counters, then the electrons and ions appended:
     // candidates, elastic, excitation, ionisation, coulomb pairs,
     // ion candidates, ion elastic, ion charge exchange
     unsigned long long* counts = nullptr;
@@ -111,9 +113,8 @@ struct CollideState {
     int* ncand = nullptr;                  // MCC candidates per cell
     int* cand_off = nullptr;               // their staging offsets
     Secondary* stage = nullptr;
-    int* flags = nullptr;
-    int* pos = nullptr;
-    int* stage_tmp = nullptr;
+    int* flags = nullptr;                  // per staging slot: 1 electron, 2 ion to append
+    int* stage_scan = nullptr;             // state of their prefix sums
     long stage_cap = 0;
     int* overflow = nullptr;                // staging or store overflow (device-driven step)
     double svmax_init = 0.0;                // initial (sigma v)_max of the electron MCC

@@ -1463,7 +1463,7 @@ uint64_t buffers_signature(const picgpu_ctx* c) {
         mix(c->coll.sel[k]);
         mix(c->coll.sel2[k]);
     }
-    const void* ps[] = {c->coll.stage, c->coll.flags, c->coll.pos, c->coll.stage_tmp, c->coll.cell_start,
+    const void* ps[] = {c->coll.stage, c->coll.flags, c->coll.stage_scan, c->coll.cell_start,
                         c->coll.cell_count, c->coll.cell_cursor, c->coll.scan_tmp, c->coll.ncand, c->coll.cand_off,
                         c->acc9, c->Ec4};
     for (const void* p : ps) mix(p);

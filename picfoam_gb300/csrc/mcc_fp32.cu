@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 
 #include "collide.h"
+#include "counts.cuh"
 
 namespace pgd {
 namespace {
@@ -94,9 +95,7 @@ __device__ __forceinline__ float at32(const Bracket32& b, float x, const float* 
     return v[b.lo] + ((x - e[b.lo]) / (e[b.hi] - e[b.lo])) * (v[b.hi] - v[b.lo]);
 }
 
-__global__ void __launch_bounds__(256) mcc_fp32_kernel(MccParams M, DSpecies el, Secondary* __restrict__ stage) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= M.n_cells) return;
+__device__ void mcc_cell32(const MccParams& M, const DSpecies& el, Secondary* __restrict__ stage, int c, u64 (&k)[4]) {
     const int eC = M.e_start[c + 1] - M.e_start[c];
     const double sv = M.svmax[c];
     const double coll = M.rem[c] + double(eC) * M.n_gas * sv * M.dt;
@@ -125,7 +124,7 @@ __global__ void __launch_bounds__(256) mcc_fp32_kernel(MccParams M, DSpecies el,
         // this cell's slots below the capacity stay unused: clear them so
         // that no stale flag is appended
         atomicExch(M.overflow, 1);
-        for (long k = base; k < long(base) + nC && k < M.stage_cap; ++k) stage[k].flag = 0;
+        for (long k = base; k < long(base) + nC && k < M.stage_cap; ++k) M.flags[k] = 0;
     }
     for (long i = 0; i < nC; ++i) {
         int j = int(uni(r) * float(eC));
@@ -198,17 +197,27 @@ __global__ void __launch_bounds__(256) mcc_fp32_kernel(MccParams M, DSpecies el,
                 sc.tet_i = sc.tet;
                 for (int a = 0; a < 3; ++a) sc.y_i[a] = sc.y[a];
             }
-            if (room) stage[base + i] = sc;
+            if (room) {
+                M.flags[base + i] = sc.flag;
+                if (sc.flag) stage[base + i] = sc;
+            }
             continue;
         }
-        if (room) stage[base + i].flag = 0;
+        if (room) M.flags[base + i] = 0;
     }
     if (sv_run > sv) M.svmax[c] = sv_run;
     if (M.iz_cell && niz) M.iz_cell[c] += niz;
-    atomicAdd(M.counts + 0, (unsigned long long)nC);
-    if (nel) atomicAdd(M.counts + 1, nel);
-    if (nex) atomicAdd(M.counts + 2, nex);
-    if (niz) atomicAdd(M.counts + 3, niz);
+    k[0] = u64(nC);
+    k[1] = nel;
+    k[2] = nex;
+    k[3] = niz;
+}
+
+__global__ void __launch_bounds__(256) mcc_fp32_kernel(MccParams M, DSpecies el, Secondary* __restrict__ stage) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    u64 k[4] = {};
+    if (c < M.n_cells) mcc_cell32(M, el, stage, c, k);
+    add_counts(M.counts, {0, 1, 2, 3}, k);
 }
 
 }  // namespace
