@@ -139,6 +139,7 @@ struct MoveParams {
     double q, mass, value;   // charge, mass, charge * weight
     double weight;
     double dt;
+    double half_dt, qdm_half, qdm_full;   // dt / 2; q (dt / 2) / m and q dt / m
     double B[3];
     double fix_scale;
     // FP32 form: the same constants pre-rounded on the host, so the kernel

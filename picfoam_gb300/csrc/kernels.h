@@ -6,7 +6,7 @@
 namespace pgd {
 
 cudaError_t move_fp64_set_tables(const TetConst& t, const PatchConst& p);
-void launch_move_fp64(const MoveParams& P, int grid, cudaStream_t s);
+void launch_move_fp64(const MoveParams& P, int sms, cudaStream_t s);
 // Returns the number of kernels launched (in-cell mover + crossing tracker, or
 // the general kernel).
 int launch_move_fp32(const MoveParams& P, int grid, cudaStream_t s);

@@ -605,6 +605,9 @@ pgd::MoveParams move_params(picgpu_ctx* c, int s, bool deposit_only) {
     P.value = S.charge * S.weight;
     P.weight = S.weight;
     P.dt = c->cfg.dt;
+    P.half_dt = 0.5 * c->cfg.dt;
+    P.qdm_half = S.charge * P.half_dt / S.mass;
+    P.qdm_full = S.charge * P.dt / S.mass;
     for (int a = 0; a < 3; ++a) P.B[a] = c->cfg.B[a];
     P.fix_scale = c->fix_scale;
     P.E = c->E;
@@ -666,13 +669,12 @@ picgpu_status move_species(picgpu_ctx* c, bool deposit_only) {
     for (int s = 0; s < c->cfg.n_species; ++s) {
         if (c->sp[s].n == 0) continue;
         const pgd::MoveParams P = move_params(c, s, deposit_only);
-        const int grid = grid_for(c, c->sp[s].n);
         {
             PhaseScope ps(c, PICGPU_PHASE_MOVE);
             if (c->mixed) {
                 c->launches += pgd::launch_move_fp32(P, 5 * c->sm_count, c->stream);
             } else {
-                pgd::launch_move_fp64(P, grid, c->stream);
+                pgd::launch_move_fp64(P, c->sm_count, c->stream);
                 c->launches++;
             }
         }
@@ -1269,7 +1271,7 @@ picgpu_status pgd_collisions(picgpu_ctx* c, picgpu_step_stats* stats) {
             if (c->mixed) {
                 c->launches += pgd::launch_move_fp32(P, 5 * c->sm_count, c->stream);
             } else {
-                pgd::launch_move_fp64(P, grid_for(c, newn[s] - old), c->stream);
+                pgd::launch_move_fp64(P, c->sm_count, c->stream);
                 c->launches++;
             }
         }
