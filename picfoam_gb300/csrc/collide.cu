@@ -223,13 +223,54 @@ __global__ void scatter_cells_kernel(const int32_t* __restrict__ tet, int n, con
     }
 }
 
-// Order every cell's list by particle index: one warp per cell; each lane
-// ranks its element against the whole list through shuffles (indices are
-// distinct), writes it to its rank in tmp, and the warp copies the list back.
+// Sorts a warp's list a[0, L), L <= 32 N, by a bitonic network over 32 N slots,
+// element e = lane + 32 r in v[r] (padding sorts last): the pairs (e, e ^ j) hold
+// (min, max) where e & k == 0, (max, min) elsewhere.
+template <int N>
+__device__ __forceinline__ void sort_list(int* a, int L, int lane) {
+    int v[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) v[r] = lane + 32 * r < L ? a[lane + 32 * r] : 0x7fffffff;
+    for (int k = 2; k <= 32 * N; k <<= 1) {
+#pragma unroll
+        for (int q = N / 2; q >= 1; q >>= 1) {   // j = 32 q: slots of the same lane
+            if (64 * q > k) continue;
+#pragma unroll
+            for (int r = 0; r < N; ++r) {
+                if (r & q) continue;
+                const int lo = min(v[r], v[r + q]), hi = max(v[r], v[r + q]);
+                const bool up = ((lane + 32 * r) & k) == 0;
+                v[r] = up ? lo : hi;
+                v[r + q] = up ? hi : lo;
+            }
+        }
+        for (int j = min(k >> 1, 16); j > 0; j >>= 1) {
+#pragma unroll
+            for (int r = 0; r < N; ++r) {
+                const int e = lane + 32 * r;
+                const int w = __shfl_xor_sync(0xffffffffu, v[r], j);
+                const bool keep_min = ((e & j) == 0) == ((e & k) == 0);
+                v[r] = keep_min ? min(v[r], w) : max(v[r], w);
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < N; ++r)
+        if (lane + 32 * r < L) a[lane + 32 * r] = v[r];
+}
+
+// Order every cell's list by particle index, one warp per cell: lists of up to
+// 32 N by a bitonic network in registers; beyond, each lane ranks its element
+// against the whole list through shuffles (indices are distinct), writes it to
+// its rank in tmp, and the warp copies the list back.  A list of 400 takes 560
+// shuffles in the network and 5200 to rank; the registers of the longest
+// network halve the warps that look for lists already in order, 50 us of a step
+// with 262,000 lists of 38.
 // With `need`, only the cells whose need is non-zero (the background MCC's
 // candidate counts, when nothing else reads the lists).
+template <int N>
 __global__ void order_cells_kernel(int n_cells, const int* __restrict__ start, int* __restrict__ idx,
-                                   int* __restrict__ tmp, const int* __restrict__ need = nullptr) {
+                                   int* __restrict__ tmp, const int* __restrict__ need) {
     const int cell = int((long(blockIdx.x) * blockDim.x + threadIdx.x) >> 5);
     const int lane = threadIdx.x & 31;
     if (cell >= n_cells) return;
@@ -243,32 +284,11 @@ __global__ void order_cells_kernel(int n_cells, const int* __restrict__ start, i
     bool sorted = true;
     for (int i = lane + 1; i < L; i += 32) sorted = sorted && a[i - 1] < a[i];
     if (__all_sync(0xffffffffu, sorted)) return;
-    if (L <= 64) {
-        // bitonic network over 64 slots, element e = lane + 32 r in v[r]
-        // (padding sorts last); pairs (e, e ^ j) hold (min, max) where
-        // e & k == 0, (max, min) elsewhere
-        int v[2] = {lane < L ? a[lane] : 0x7fffffff, lane + 32 < L ? a[lane + 32] : 0x7fffffff};
-        for (int k = 2; k <= 64; k <<= 1) {
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                if (j == 32) {
-                    const int lo = min(v[0], v[1]), hi = max(v[0], v[1]);
-                    const bool up = (lane & k) == 0;
-                    v[0] = up ? lo : hi;
-                    v[1] = up ? hi : lo;
-                } else {
-#pragma unroll
-                    for (int r = 0; r < 2; ++r) {
-                        const int e = lane + 32 * r;
-                        const int w = __shfl_xor_sync(0xffffffffu, v[r], j);
-                        const bool keep_min = ((e & j) == 0) == ((e & k) == 0);
-                        v[r] = keep_min ? min(v[r], w) : max(v[r], w);
-                    }
-                }
-            }
-        }
-        if (lane < L) a[lane] = v[0];
-        if (lane + 32 < L) a[lane + 32] = v[1];
-        return;
+    if (L <= 64) return sort_list<2>(a, L, lane);
+    if constexpr (N == 16) {
+        if (L <= 128) return sort_list<4>(a, L, lane);
+        if (L <= 256) return sort_list<8>(a, L, lane);
+        if (L <= 512) return sort_list<16>(a, L, lane);
     }
     for (int base = 0; base < L; base += 32) {
         const int i = base + lane;
@@ -285,7 +305,15 @@ __global__ void order_cells_kernel(int n_cells, const int* __restrict__ start, i
     for (int i = lane; i < L; i += 32) a[i] = t[i];
 }
 
-unsigned order_blocks(int n_cells) { return unsigned((long(n_cells) * 32 + 255) / 256); }
+// The network by the mean length of a list (n parcels): the short one while
+// few lists are longer than its 64 slots.
+void launch_order(int n_cells, long n, const int* start, int* idx, int* tmp, const int* need, cudaStream_t s,
+                  int64_t* launches) {
+    const unsigned blocks = unsigned((long(n_cells) * 32 + 255) / 256);
+    if (n <= 48L * n_cells) order_cells_kernel<2><<<blocks, 256, 0, s>>>(n_cells, start, idx, tmp, need);
+    else order_cells_kernel<16><<<blocks, 256, 0, s>>>(n_cells, start, idx, tmp, need);
+    *launches += 1;
+}
 
 // ------------------------------------------------------------- Philox ---
 struct Rng {
@@ -1249,6 +1277,22 @@ __device__ __forceinline__ double warp_tree_sum(double v) {
     return __shfl_sync(0xffffffffu, v, 0);
 }
 
+// The sum of n terms, given by `term` or, where no parcel has a weight of its
+// own (nw null), all equal to `same`: one product; else the lanes' partial sums
+// in the tree.  Summed by lane 0 parcel by parcel, the weights of a cell of
+// 2 x 400 were almost half of the Coulomb kernel's FP64 instructions.
+template <class F>
+__device__ __forceinline__ double warp_sum(int n, const double* nw, double same, int lane, F term) {
+    if (!nw) return double(n) * same;
+    double v = 0.0;
+    for (int t = lane; t < n; t += 32) v += term(t);
+    return warp_tree_sum(v);
+}
+
+__device__ __forceinline__ const double* own_weights(const CoulombSpecies& C, int a, int b) {
+    return C.p[a].nw ? C.p[a].nw : C.p[b].nw;
+}
+
 template <class R>
 __device__ double debye_length_warp(const CoulombSpecies& C, const CoulombParams& K, int c, int lane) {
     double debye = 0.0, n_max = 0.0;
@@ -1570,17 +1614,11 @@ __global__ void __launch_bounds__(32 * kCoulombWarps) coulomb_kernel(CoulombSpec
             const int nA = C.start[a][c + 1] - sa, nB = C.start[b][c + 1] - sb;
             const int* LA = C.idx[a] + sa;
             const int* LB = C.idx[b] + sb;
-            // NanbuYonemuraPairing.C:96-113: the real particles of each
-            // species, parcel by parcel in list order (lane 0)
+            // NanbuYonemuraPairing.C:96-113: the real particles of each species
             double sA = 0.0, sB = 0.0;
             if (!K.takizuka_abe) {
-                if (lane == 0) {
-                    for (int t = 0; t < nA; ++t) sA += pweight(C, a, LA[t]);
-                    if (a != b)
-                        for (int t = 0; t < nB; ++t) sB += pweight(C, b, LB[t]);
-                }
-                sA = __shfl_sync(0xffffffffu, sA, 0);
-                sB = __shfl_sync(0xffffffffu, sB, 0);
+                sA = warp_sum(nA, C.p[a].nw, C.w[a], lane, [&](int t) { return pweight(C, a, LA[t]); });
+                if (a != b) sB = warp_sum(nB, C.p[b].nw, C.w[b], lane, [&](int t) { return pweight(C, b, LB[t]); });
             }
             if (a == b && nA > 1) {
                 if (!K.allow_intra) continue;
@@ -1625,14 +1663,11 @@ __global__ void __launch_bounds__(32 * kCoulombWarps) coulomb_kernel(CoulombSpec
                     // collision follows the first one's on parcel sel[0]
                     // NanbuYonemuraPairing.C:128-141: real particles that
                     // collide, the extra pair first
-                    double nAA = 0.0;
-                    if (lane == 0) {
-                        nAA += 2.0 * fmin(pweight(C, a, LA[sel[nA - 1]]), pweight(C, a, LA[sel[0]]));
-                        for (int x = 0; x < nA - 2; x += 2)
-                            nAA += 2.0 * fmin(pweight(C, a, LA[sel[x]]), pweight(C, a, LA[sel[x + 1]]));
-                    }
-                    const double n12 = __shfl_sync(0xffffffffu, nAA, 0) / V;
                     const int np = (nA - 1) / 2;
+                    const double n12 = warp_sum(np + 1, C.p[a].nw, 2.0 * C.w[a], lane, [&](int x) {
+                        const int P = x < np ? 2 * x : nA - 1, Q = x < np ? 2 * x + 1 : 0;
+                        return 2.0 * fmin(pweight(C, a, LA[sel[P]]), pweight(C, a, LA[sel[Q]]));
+                    }) / V;
                     for (int x = lane; x < np; x += 32) {
                         Rng r = cs.collision(ord + x);
                         collide<R>(C, K, a, LA[sel[2 * x]], a, LA[sel[2 * x + 1]], lD, n, n, n12, r);
@@ -1644,12 +1679,10 @@ __global__ void __launch_bounds__(32 * kCoulombWarps) coulomb_kernel(CoulombSpec
                     ord += np + 1;
                     pairs += 1 + nA / 2;
                 } else {
-                    double nAA = 0.0;
-                    if (lane == 0)
-                        for (int x = 0; x < nA - 1; x += 2)
-                            nAA += 2.0 * fmin(pweight(C, a, LA[sel[x]]), pweight(C, a, LA[sel[x + 1]]));
-                    const double n12 = __shfl_sync(0xffffffffu, nAA, 0) / V;
                     const int np = nA / 2;
+                    const double n12 = warp_sum(np, C.p[a].nw, 2.0 * C.w[a], lane, [&](int x) {
+                        return 2.0 * fmin(pweight(C, a, LA[sel[2 * x]]), pweight(C, a, LA[sel[2 * x + 1]]));
+                    }) / V;
                     for (int x = lane; x < np; x += 32) {
                         Rng r = cs.collision(ord + x);
                         collide<R>(C, K, a, LA[sel[2 * x]], a, LA[sel[2 * x + 1]], lD, n, n, n12, r);
@@ -1672,18 +1705,18 @@ __global__ void __launch_bounds__(32 * kCoulombWarps) coulomb_kernel(CoulombSpec
                         nQ = sB / V;
                         nPQ = 0.0;
                     }
-                    // the pairs' real particles and the ionisation densities
-                    // (initIonization, prepareNumberDensities), lane 0 in order
-                    double nAB = 0.0;
-                    if (lane == 0) {
-                        if (Z.on) perez_init(Z, a, b, nP, nQ, np, ne, nei);
-                        for (int k = 0; k < nA; ++k) {
-                            if (!K.takizuka_abe)
-                                nAB += fmin(pweight(C, a, LA[sel[k]]), pweight(C, b, LB[sel[nA - k - 1]]));
-                            if (Z.on) perez_densities<R>(C, Z, a, LA[sel[k]], b, LB[sel[nA - k - 1]], ne, nei);
-                        }
+                    // the pairs' real particles
+                    if (!K.takizuka_abe)
+                        nPQ = warp_sum(nA, own_weights(C, a, b), fmin(C.w[a], C.w[b]), lane, [&](int k) {
+                            return fmin(pweight(C, a, LA[sel[k]]), pweight(C, b, LB[sel[nA - k - 1]]));
+                        }) / V;
+                    // the ionisation densities (initIonization,
+                    // prepareNumberDensities), lane 0 in order
+                    if (lane == 0 && Z.on) {
+                        perez_init(Z, a, b, nP, nQ, np, ne, nei);
+                        for (int k = 0; k < nA; ++k)
+                            perez_densities<R>(C, Z, a, LA[sel[k]], b, LB[sel[nA - k - 1]], ne, nei);
                     }
-                    if (!K.takizuka_abe) nPQ = __shfl_sync(0xffffffffu, nAB, 0) / V;
                     np = __shfl_sync(0xffffffffu, np, 0);
                     ne = __shfl_sync(0xffffffffu, ne, 0);
                     nei = __shfl_sync(0xffffffffu, nei, 0);
@@ -1769,16 +1802,16 @@ __global__ void __launch_bounds__(32 * kCoulombWarps) coulomb_kernel(CoulombSpec
                     }
                     const double nMaxS = (maxS == a ? sA : sB) / V;
                     const double nMinS = (maxS == a ? sB : sA) / V;
-                    double nAB = 0.0;
-                    if (lane == 0) {
-                        if (Z.on) perez_init(Z, minS, maxS, nMinS, nMaxS, np, ne, nei);
+                    const double n12 = warp_sum(nMax, own_weights(C, a, b), fmin(C.w[a], C.w[b]), lane, [&](int l) {
+                        return fmin(pweight(C, minS, Lmin[smin[l % nMin]]), pweight(C, maxS, Lmax[smax[l]]));
+                    }) / V;
+                    if (lane == 0 && Z.on) {
+                        perez_init(Z, minS, maxS, nMinS, nMaxS, np, ne, nei);
                         for (int l = 0, k = 0; l < nMax; ++l, ++k) {
                             if (k >= nMin) k = 0;
-                            nAB += fmin(pweight(C, minS, Lmin[smin[k]]), pweight(C, maxS, Lmax[smax[l]]));
-                            if (Z.on) perez_densities<R>(C, Z, minS, Lmin[smin[k]], maxS, Lmax[smax[l]], ne, nei);
+                            perez_densities<R>(C, Z, minS, Lmin[smin[k]], maxS, Lmax[smax[l]], ne, nei);
                         }
                     }
-                    const double n12 = __shfl_sync(0xffffffffu, nAB, 0) / V;
                     np = __shfl_sync(0xffffffffu, np, 0);
                     ne = __shfl_sync(0xffffffffu, ne, 0);
                     nei = __shfl_sync(0xffffffffu, nei, 0);
@@ -2508,10 +2541,7 @@ int occupancy(CollideState& st, const CollideArgs& a, int s, std::string* msg, i
         scatter_cells_kernel<<<grid_of(n, 256), 256, 0, a.stream>>>(a.sp[s].tet, int(n), start, st.cell_cursor,
                                                                     st.idx[s]);
         *launches += 1;
-        if (ordered) {
-            order_cells_kernel<<<order_blocks(nc), 256, 0, a.stream>>>(nc, start, st.idx[s], st.sel[s]);
-            *launches += 1;
-        }
+        if (ordered) launch_order(nc, n, start, st.idx[s], st.sel[s], nullptr, a.stream, launches);
     }
     return cudaGetLastError() == cudaSuccess ? PICGPU_OK : PICGPU_CUDA_ERROR;
 }
@@ -3003,11 +3033,8 @@ int run_collisions(CollideState& st, const CollideArgs& a, int64_t counts[kColli
         MccParams M = mcc_setup(st, a);
         // candidates per cell and their staging offsets
         mcc_count_kernel<<<(nc + 255) / 256, 256, 0, a.stream>>>(M, st.ncand);
-        if (mcc_only) {
-            order_cells_kernel<<<order_blocks(nc), 256, 0, a.stream>>>(nc, M.e_start, st.idx[es], st.sel[es],
-                                                                       st.ncand);
-            *launches += 1;
-        }
+        if (mcc_only)
+            launch_order(nc, a.n[es], M.e_start, st.idx[es], st.sel[es], st.ncand, a.stream, launches);
         exclusive_scan(st.ncand, st.cand_off, nc, st.scan_tmp, st.overflow, a.stream, launches);
         int total = 0;
         cudaMemcpyAsync(&total, st.cand_off + nc, sizeof(int), cudaMemcpyDeviceToHost, a.stream);
@@ -3128,10 +3155,7 @@ int run_collisions_device(CollideState& st, const CollideArgs& a, int* n_dev, in
         scatter_cells_kernel<<<grid_of(cap, 256), 256, 0, a.stream>>>(a.sp[s].tet, int(cap), start, st.cell_cursor,
                                                                       st.idx[s], n_dev + s);
         *launches += 2;
-        if (!mcc_lists_only(cfg)) {
-            order_cells_kernel<<<order_blocks(nc), 256, 0, a.stream>>>(nc, start, st.idx[s], st.sel[s]);
-            *launches += 1;
-        }
+        if (!mcc_lists_only(cfg)) launch_order(nc, a.n[s], start, st.idx[s], st.sel[s], nullptr, a.stream, launches);
     }
     if (cfg.coulomb.enabled) {
         CoulombSpecies C;
@@ -3149,11 +3173,8 @@ int run_collisions_device(CollideState& st, const CollideArgs& a, int* n_dev, in
         M.step_dev = step_dev;
         const long scap = st.stage_cap;
         mcc_count_kernel<<<(nc + 255) / 256, 256, 0, a.stream>>>(M, st.ncand);
-        if (mcc_lists_only(cfg)) {
-            order_cells_kernel<<<order_blocks(nc), 256, 0, a.stream>>>(nc, M.e_start, st.idx[es], st.sel[es],
-                                                                       st.ncand);
-            *launches += 1;
-        }
+        if (mcc_lists_only(cfg))
+            launch_order(nc, a.n[es], M.e_start, st.idx[es], st.sel[es], st.ncand, a.stream, launches);
         exclusive_scan(st.ncand, st.cand_off, nc, st.scan_tmp, st.overflow, a.stream, launches);
         if (a.mixed && !M.relativistic && M.xs32) launch_mcc_fp32(M, a.sp[es], st.stage, st.mcc_block, a.stream);
         else if (a.mixed) mcc_kernel<float><<<(nc + st.mcc_block - 1) / st.mcc_block, st.mcc_block, 0, a.stream>>>(M, a.sp[es], st.stage);
