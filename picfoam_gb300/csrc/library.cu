@@ -672,7 +672,7 @@ picgpu_status move_species(picgpu_ctx* c, bool deposit_only) {
         {
             PhaseScope ps(c, PICGPU_PHASE_MOVE);
             if (c->mixed) {
-                c->launches += pgd::launch_move_fp32(P, 5 * c->sm_count, c->stream);
+                c->launches += pgd::launch_move_fp32(P, pgd::kMoveBlocks32 * c->sm_count, c->stream);
             } else {
                 pgd::launch_move_fp64(P, c->sm_count, c->stream);
                 c->launches++;
@@ -1269,7 +1269,7 @@ picgpu_status pgd_collisions(picgpu_ctx* c, picgpu_step_stats* stats) {
             pgd::MoveParams P = move_params(c, s, true);
             P.first = int(old);
             if (c->mixed) {
-                c->launches += pgd::launch_move_fp32(P, 5 * c->sm_count, c->stream);
+                c->launches += pgd::launch_move_fp32(P, pgd::kMoveBlocks32 * c->sm_count, c->stream);
             } else {
                 pgd::launch_move_fp64(P, c->sm_count, c->stream);
                 c->launches++;

@@ -422,7 +422,7 @@ __device__ __forceinline__ void deposit32(const MoveParams& P, const unsigned* t
 // address), then the 8 corner slots; the flush adds the copies.
 constexpr int kCellSub = 4;
 constexpr int kCellSlots = kCellSub + 8;
-constexpr int kCellWindow = 768;
+constexpr int kCellWindow = 512;
 
 __device__ __forceinline__ void deposit_cell32(const MoveParams& P, const unsigned* tri_of, const S32& s, int w0,
                                                unsigned* win) {
@@ -936,7 +936,7 @@ int launch_pusher(const MoveParams& P, int blocks, int chunk, bool cell, cudaStr
 
 }  // namespace
 
-// grid: the number of resident blocks to use (5 per SM); each block takes one
+// grid: the number of blocks to use (5 per SM are resident); each block takes one
 // contiguous chunk (a multiple of 256 particles) of [P.first, P.n).  With
 // P.n_dev set the counts are read on the device and all grid blocks launch.
 // Uniform block meshes with a crossing queue run the in-cell mover and the
