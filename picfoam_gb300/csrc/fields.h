@@ -19,8 +19,9 @@ struct PcgState {
     double rz, rr, bb, pq, beta, lim, mean, of_residual, alpha;
     int done, iters, converged, k;
     unsigned int ticket;
-    // persistent solve (pcg.cu): wait counters, blocks gone, a wait ran out
-    unsigned int bar[3], exits;
+    // persistent solve (pcg.cu): number of its last pass, arrivals, blocks gone,
+    // a wait ran out
+    unsigned int pass, bar[5], exits;
     int fail;
     double rr0;   // r.r of the start guess
 };
@@ -36,10 +37,17 @@ struct PcgPlan {
     bool fits = false;  // every block resident at once: the persistent solve runs
 };
 cudaError_t pcg_make_plan(int n, bool uniform, PcgPlan* plan);
-// The whole solve M x = b from the given x in one launch; u holds n doubles,
-// part 4 x pcg_blocks(n); st must be zero but for mean before the first solve
-// and after one that set st->fail.
-cudaError_t launch_pcg_solve(const DMesh& m, const PcgPlan& plan, const double* b, double* x, double* u, double* part,
+// A value that blocks of the persistent solve exchange: its halves, each with
+// the number of the pass it belongs to in the upper 32 bits.
+struct alignas(16) PcgSlot {
+    unsigned long long lo, hi;
+};
+int pcg_blocks(int n);
+inline long pcg_slots(int n) { return 2 * long(n) + 8 * long(pcg_blocks(n)); }
+// The whole solve M x = b from the given x in one launch.  slots
+// (pcg_slots(n)) and, but for mean, st must be zero before the first solve and
+// after one that set st->fail, and are kept between solves of the same size.
+cudaError_t launch_pcg_solve(const DMesh& m, const PcgPlan& plan, const double* b, double* x, PcgSlot* slots,
                              PcgState* st, double tol, int maxit, cudaStream_t s);
 
 // q * weight * 2^-kDepositBits per species (the FP32 form's fixed-point deposit).

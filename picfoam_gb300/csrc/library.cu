@@ -315,6 +315,7 @@ struct picgpu_ctx {
     cudaEvent_t timer[2] = {nullptr, nullptr};
     cudaGraphExec_t pcg_graph = nullptr;   // beyond the persistent solve's size
     pgd::PcgPlan pcg_plan;
+    pgd::PcgSlot* pcg_slots = nullptr;          // its exchange between blocks
     double pcg_r0 = 0.0;  // ||b - A x0|| / ||b|| of the last solve's start guess
     std::unique_ptr<pgd::LearnedWarmStart> ws;  // learned warm start (cfg.learned.enabled)
     std::unique_ptr<pgd::MultigridPCG> mg;      // multigrid-preconditioned PCG (cfg.pcg_precond)
@@ -781,7 +782,7 @@ picgpu_status poisson(picgpu_ctx* c, picgpu_step_stats* stats, bool learned = fa
             c->st_host->bb = bb;
             c->st_host->converged = conv ? 1 : 0;
         } else if (c->pcg_plan.fits) {
-            CK(pgd::launch_pcg_solve(c->dm, c->pcg_plan, c->b, c->phi, c->z, c->part, c->st, tol, maxit, c->stream));
+            CK(pgd::launch_pcg_solve(c->dm, c->pcg_plan, c->b, c->phi, c->pcg_slots, c->st, tol, maxit, c->stream));
             pgd::launch_of_residual(c->dm, c->b, c->phi, c->part, c->st, c->stream);
             c->launches += 3;
             CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
@@ -817,6 +818,7 @@ picgpu_status poisson(picgpu_ctx* c, picgpu_step_stats* stats, bool learned = fa
     if (!c->mg && c->pcg_plan.fits) {
         if (S.fail) {
             CK(cudaMemset(c->st, 0, sizeof(pgd::PcgState)));
+            CK(cudaMemset(c->pcg_slots, 0, sizeof(pgd::PcgSlot) * pgd::pcg_slots(c->m.n_cells)));
             return bad(c, PICGPU_CUDA_ERROR, "Poisson PCG: a block of the solver kernel waited too long for the others");
         }
         c->pcg_r0 = S.bb > 0 ? std::sqrt(S.rr0 / S.bb) : 0.0;
@@ -1965,6 +1967,11 @@ static picgpu_status create_with_mesh(picgpu_ctx* c, const picgpu_config* cfg) {
     }
     CK(cudaMemset(c->st, 0, sizeof(pgd::PcgState)));
     CK(pgd::pcg_make_plan(int(nc), c->dm.lap_uniform != 0, &c->pcg_plan));
+    if (c->pcg_plan.fits) {
+        const size_t slots = size_t(pgd::pcg_slots(int(nc)));
+        if ((s = dalloc(c, &c->pcg_slots, slots))) return s;
+        CK(cudaMemset(c->pcg_slots, 0, slots * sizeof(pgd::PcgSlot)));
+    }
     CK(cudaMallocHost(&c->st_host, sizeof(pgd::PcgState)));
     CK(cudaMallocHost(&c->counters_host, sizeof(pgd::MoveCounters) * PICGPU_MAX_SPECIES));
     std::memset(c->st_host, 0, sizeof(pgd::PcgState));

@@ -21,22 +21,37 @@
 // What bounds it: on this part one FP64 warp instruction holds its quarter of
 // the SM for 64 cycles (a dependent chain costs the same, a division 580), so
 // a chunk's iteration keeps one SM busy for 8192 cycles, and on small meshes
-// the chain "all u written - SpMV - sum of delta - one division - update"
-// with its two waits for all blocks counts.  Hence
+// the chain "u of the neighbours - SpMV - sum of delta - one division - update"
+// counts, which goes through L2 twice (a store seen by a load elsewhere: some
+// 1400 cycles).  Hence
 //   * one cooperative launch per solve: r, p, s, w, u of a cell stay with its
 //     thread (registers; shared memory when a block has several chunks) and
 //     only u and the chunk sums pass through L2;
+//   * blocks do not meet: a value that passes through L2 carries the number of
+//     its pass (PcgSlot), and who needs it reads it until the number is right.
+//     Counting arrivals instead (all written, fence, atomic, poll, then the
+//     load of the value) took three trips more per iteration.  Two sets of
+//     slots, used in turn: a set is written again two passes later, when the
+//     sums of the pass between, to which every block adds after its reads,
+//     are known;
 //   * a cluster of 2 to 8 blocks shares a chunk when the chunks alone would
 //     leave SMs idle, one cell per thread so that all four quarters of an SM
-//     work; the chunk's tree reads its sums through distributed shared memory;
+//     work; the blocks send their thread sums to the block that adds them up
+//     (st.async into its shared memory, counted by an mbarrier);
 //   * three further warps per block hold everything that is not per cell:
 //     one forms gamma, beta and beta gamma / alpha_old (two of the three
-//     divisions), one r.r, while the others run the SpMV; the third waits for
-//     the other blocks and closes the iteration with delta and alpha;
+//     divisions), one r.r, while the others run the SpMV; the third closes the
+//     iteration with delta and alpha;
 //   * x, p and s are updated while delta is summed.
-// Per iteration on GB300, against the two-kernel iteration of fields.cu in a
-// CUDA graph: 128 cells 2 (11.5) us, 5917 cells 6.6 (18.6), 27,000 cells
-// 6.8 (19), 91,125 cells 9.5 (19.5), 262,144 cells 16.0 (21).
+// A block with whole chunks has 6144 neighbours to read per chunk, which as
+// slots are twice the bytes: there u is exchanged as it is behind an arrival
+// counter, and with one chunk per block, where the registers are full, so are
+// the sums of the chunks.
+// Per iteration on GB300 (before: with arrival counters throughout, and as the
+// two-kernel iteration of fields.cu in a CUDA graph): 5917 cells 4.2 us (6.4,
+// 18.6), 27,000 cells 5.5 (7.2, 19), 64,000 cells 6.9 (8.1), 91,125 cells 9.0
+// (9.3, 19.5; 10.0 with slots), 262,144 cells 15.8 (15.7, 21; 18.4 with slots
+// for u), 512,000 cells 25.3 (27.4); one block of 128 cells 2 us (2, 11.5).
 #include "fields.h"
 #include "reduce.cuh"
 
@@ -62,8 +77,8 @@ struct PcgArgs {
     DMesh m;
     const double* __restrict__ b;
     double* x;
-    double* u;          // exchanged between blocks
-    double* part;       // gamma, r.r, delta, b.b sums of the chunks
+    PcgSlot* u;         // exchanged between blocks: two sets of n
+    PcgSlot* part;      // gamma, r.r, delta, b.b sums of the chunks, two sets each
     PcgState* st;
     double tol;
     int maxit;
@@ -89,43 +104,80 @@ struct Store<kSmem, I> {
     __device__ double& x(int, long c) { return xg[c]; }
 };
 
-__device__ __forceinline__ void arrive(unsigned* bar) {
-    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+using u64 = unsigned long long;
+
+// A slot's two words each hold half of the value and the pass number, so each
+// is valid by itself whatever order the words arrive in.
+__device__ __forceinline__ void put_slot(PcgSlot* p, double v, unsigned pass) {
+    const u64 b = u64(__double_as_longlong(v)), e = u64(pass) << 32;
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"((b & 0xffffffffull) | e), "l"((b >> 32) | e)
+                 : "memory");
+}
+__device__ __forceinline__ bool get_slot(const PcgSlot* p, unsigned pass, double* v) {
+    u64 lo, hi;
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "l"(p) : "memory");
+    *v = __longlong_as_double((long long)((lo & 0xffffffffull) | (hi << 32)));
+    return unsigned(lo >> 32) == pass && unsigned(hi >> 32) == pass;
 }
 
-// Waits until the counter has passed `target`; false when the poll limit ran out.
-__device__ __forceinline__ bool wait(const unsigned* bar, unsigned target) {
-    for (unsigned i = 0; i < kSpinLimit; ++i) {
-        unsigned v;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-        if (int(v - target) >= 0) return true;
+__device__ __forceinline__ bool get(const PcgSlot* p, unsigned pass, double* v) { return get_slot(p, pass, v); }
+__device__ __forceinline__ bool get(const double* p, unsigned, double* v) {
+    *v = __ldcg(p);
+    return true;
+}
+
+// Repeats ready() (uniform over the warp) until it holds; false when the limit
+// ran out or another block gave up.
+template <class F>
+__device__ __forceinline__ bool wait_for(F ready, unsigned limit, const int* fail) {
+    for (unsigned i = 1; i < limit; ++i) {
+        if (ready()) return true;
+        if ((i & 1023u) == 0 && *static_cast<const volatile int*>(fail)) break;
     }
     return false;
 }
 
+__device__ __forceinline__ unsigned smem(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
+__device__ __forceinline__ unsigned peer(unsigned addr, int rank) {
+    unsigned r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+    return r;
+}
+
+// Chunk sums that a lane reads at once, and so the chunks of a split plan.
+constexpr int sums_per_lane(int S) { return S == 8 ? 1 : S == 4 ? 2 : S == 2 ? 3 : 8; }
+
 // One warp: the sum over nb chunk sums in the order of final_sum +
 // block_tree, without the additions of zeros (which change nothing); valid in
-// every lane.
-__device__ __forceinline__ double warp_final_sum(const double* part, int nb) {
+// every lane.  *ok turns false when a sum did not come.
+template <int K, class Part>
+__device__ __forceinline__ double warp_final_sum(const Part* part, int nb, unsigned pass, const int* fail, bool* ok) {
     const int lane = threadIdx.x & 31;
-    double v[8];
+    double v[K];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = 0.0;
+    for (int k = 0; k < K; ++k) v[k] = 0.0;
     for (int i0 = 0; i0 < nb; i0 += 256) {
-        double p[8];
+        double p[K];
+        *ok = *ok && wait_for(
+                         [&] {
+                             bool all = true;
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int i = i0 + 32 * k + lane;
-            p[k] = i < nb ? __ldcg(part + i) : 0.0;
-        }
+                             for (int k = 0; k < K; ++k) {
+                                 const int i = i0 + 32 * k + lane;
+                                 p[k] = 0.0;
+                                 if (i < nb) all = get(part + i, pass, &p[k]) && all;
+                             }
+                             return sizeof(Part) == sizeof(double) || __all_sync(0xffffffffu, all);
+                         },
+                         kSpinLimit, fail);
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
+        for (int k = 0; k < K; ++k)
             if (i0 == 0) v[k] = p[k];
             else if (i0 + 32 * k < nb) v[k] = v[k] + p[k];
     }
     double r = v[0];
 #pragma unroll
-    for (int k = 1; k < 8; ++k)
+    for (int k = 1; k < K; ++k)
         if (32 * k < nb) r = r + v[k];
 #pragma unroll
     for (int off = 16; off >= 1; off >>= 1)
@@ -133,20 +185,13 @@ __device__ __forceinline__ double warp_final_sum(const double* part, int nb) {
     return __shfl_sync(0xffffffffu, r, 0);
 }
 
-// One warp: a chunk's sum from its thread sums, in the order of block_tree;
-// they lie in the S blocks of the cluster, 256 / S each, and those from
-// `count` on are zero.
-template <int S>
-__device__ __forceinline__ double warp_chunk_sum(double* tv, int count, const cg::cluster_group& cl) {
-    constexpr int per = 256 / S;
+// One warp: a chunk's sum from its 256 thread sums, in the order of
+// block_tree; those from `count` on are zero.
+__device__ __forceinline__ double warp_chunk_sum(const double* tv, int count) {
     const int lane = threadIdx.x & 31;
     double v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const int t = 32 * k + lane;
-        v[k] = 0.0;
-        if (32 * k < count) v[k] = S == 1 ? tv[t] : *cl.map_shared_rank(tv + t % per, 32 * k / per);
-    }
+    for (int k = 0; k < 8; ++k) v[k] = 32 * k < count ? tv[32 * k + lane] : 0.0;
     double r = v[0];
 #pragma unroll
     for (int k = 1; k < 8; ++k)
@@ -174,12 +219,11 @@ __device__ __forceinline__ double row(const DMesh& m, double diag, double xc, co
 }
 
 struct Scalars {
-    double g, rr, bb, beta, t, alpha, rz, lim;
-    int fail;
+    double g, rr, beta, t, alpha;
 };
 
 // Named barriers (0 is __syncthreads).
-enum { kBarU = 1, kBarW = 2, kBarT = 3, kBarBeta = 4, kBarMain = 5 };
+enum { kBarG = 1, kBarW = 2, kBarT = 3, kBarBeta = 4, kBarMain = 5, kBarU = 6 };
 __device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
 __device__ __forceinline__ void bar_arrive(int id, int n) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
@@ -191,9 +235,16 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 template <bool Uniform, int Mode, int I, int S>
 __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
     extern __shared__ double dyn[];   // sums; then kSmem: the vectors, I = 1: r, u, w of the block
-    __shared__ Scalars sc;
+    __shared__ Scalars scalars[2];    // in turn: a warp may still read one pass's while the next one's are written
+    __shared__ double sc_rz, sc_bb, sc_lim;
+    __shared__ __align__(8) u64 bars[4][2];   // S > 1: bytes received, per quantity, odd and even passes
     const cg::cluster_group cl = cg::this_cluster();
     constexpr bool alone = I == 1 && S == 1;   // one block, at most 256 cells
+    // whole chunks per block: u as it is, an arrival counter instead of slots
+    constexpr bool counted = I > 1;
+    // one chunk per block, in registers: so are the chunks' sums
+    constexpr bool counted_sums = counted && Mode == kReg;
+    constexpr int kWarpsG = counted ? 96 : 64;   // threads that wait for the block's u, gamma and r.r sums
     constexpr int per = 256 / S;
     const int M = alone ? int(blockDim.x) - kScalarThreads : threads_of(I, S) - kScalarThreads;
     const int tid = threadIdx.x;
@@ -204,19 +255,22 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
     const int slots = (A.chunks + clusters - 1) / clusters;   // chunks per block, at most
     const int nb = A.chunks, n = A.m.n_cells;
     const bool single = alone || clusters == 1;
-    unsigned ph = 0;                                     // passes begun: waits per counter
-    // sums of quantity q (0 gamma, 1 r.r, 2 delta, 3 b.b) of the block's chunk
-    // lc; gamma and r.r in two sets, as warps G and R of another block may
-    // still read one while the next is written
+    PcgState* st = A.st;
+    const unsigned pass0 = st->pass;    // number of the last solve's last pass
+    unsigned ph = 0;                    // passes begun
+    bool bad = false;                   // a wait of this thread ran out
+    // thread sums of quantity q (0 gamma, 1 r.r, 2 delta, 3 b.b) of the block's
+    // chunk lc; S > 1: what the blocks of the cluster sent.  In two sets where
+    // one may still be read while the next is written
     auto tv = [&](int q, int lc, unsigned pass) {
-        return dyn + ((q < 2 ? 2 * q + int(pass & 1u) : q + 2) * slots + lc) * per;
+        return S > 1 ? dyn + 256 * (2 * q + int(pass & 1u))
+                     : dyn + ((q < 2 ? 2 * q + int(pass & 1u) : q + 2) * slots + lc) * 256;
     };
-    double* const vals = dyn + kSums * slots * per;   // I = 1: kItems x per values of r, u, w (b)
+    double* const vals = dyn + (S > 1 ? 8 : kSums * slots) * 256;   // I = 1: kItems x per values of r, u, w (b)
     // cell of item j of this thread in chunk ch
     auto cell = [&](int ch, int j) {
         return long(ch) * kChunk + (I == 1 ? rank * per + tid % per + 256 * (tid / per) : tid + 256 * j);
     };
-    PcgState* st = A.st;
 
     Store<Mode, I> V;
     if constexpr (Mode == kSmem) {
@@ -229,21 +283,36 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
     for (int j = 0; j < I; ++j)
 #pragma unroll
         for (int f = 0; f < 6; ++f) nbr[j][f] = -1;
-    if (tid == 0) sc.fail = 0;
+    // arms the barrier of quantity q and the pass's parity
+    auto expect = [&](int q, unsigned pass) {
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem(&bars[q][pass & 1u])),
+                     "r"(256 * 8)
+                     : "memory");
+    };
+    if (S > 1) {
+        if (tid < 8) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem(&bars[tid / 2][tid % 2])) : "memory");
+            asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+            expect(tid / 2, unsigned(tid));
+        }
+        cl.sync();
+    }
     auto load_cell = [&](long c, int j) {
         dinv[j] = A.m.dinv[c];
         diag[j] = A.m.Mdiag[c];
 #pragma unroll
         for (int f = 0; f < 6; ++f) nbr[j][f] = A.m.nbr[6 * c + f];
     };
+    // u of the pass ph + 1
     auto put_u = [&](long c, int j, double v) {
         if (alone) vals[M + c] = v;
-        else __stcg(A.u + c, v);
+        else if (counted) __stcg(reinterpret_cast<double*>(A.u) + c, v);
+        else put_slot(A.u + long((ph + 1) & 1u) * n + c, v, pass0 + ph + 1);
     };
-    auto get_u = [&](long i) { return alone ? vals[M + i] : __ldcg(A.u + i); };
     constexpr int kNext = alone ? 0 : per / 32;   // first warp of the next chain
     // I = 1: sum q of strided cells t, t + 256, ... from the block's values
-    // a and b, by the warps starting at `first`
+    // a and b, by the warps starting at `first`; S > 1: sent to the block that
+    // adds the chunk up, or to all of them when there is no other chunk
     auto chain = [&](int q, const double* a, const double* b, int first) {
         const int t = tid - 32 * first;
         if (t < 0 || t >= per) return;
@@ -252,41 +321,86 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
         for (int j = 0; j < kItems; ++j)
             if (!(alone && j > 0) && long(cluster) * kChunk + rank * per + t + 256 * j < n)
                 v = fma(a[j * per + t], b[j * per + t], v);
-        tv(q, 0, ph)[t] = v;
-    };
-    auto sync_all = [&]() {
-        if (S == 1) __syncthreads();
-        else cl.sync();
+        if constexpr (S == 1) {
+            tv(q, 0, ph)[t] = v;
+        } else {
+            const unsigned to = smem(tv(q, 0, ph) + rank * per + t), bar = smem(&bars[q][ph & 1u]);
+            for (int r = 0; r < (single ? S : 1); ++r)
+                asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(
+                                 peer(to, r)),
+                             "l"(__double_as_longlong(v)), "r"(peer(bar, r))
+                             : "memory");
+        }
     };
     auto failed = [&]() {
-        // every block of the cluster learns of it before its next sync_all
-        for (int q = 0; q < S; ++q) *(S == 1 ? &sc.fail : cl.map_shared_rank(&sc.fail, q)) = 1;
-        atomicMax(&st->fail, 1);
+        bad = true;
+        if (lane == 0) atomicMax(&st->fail, 1);
     };
-    // the chunk sums of quantity q, by the calling warp
-    auto publish = [&](int q, double* out, unsigned pass) {
-        if (rank != 0) return;
-        int lc = 0;
-        for (int ch = cluster; ch < nb; ch += clusters, ++lc) {
-            const double v = warp_chunk_sum<S>(tv(q, lc, pass), min(n - ch * kChunk, 256), cl);
-            if (lane == 0) out[ch] = v;
-        }
+    // S > 1, the calling warp: the pass's sums of quantity q are there.  Its
+    // barrier is armed again at once, for two passes later: no block sends
+    // those before every block has sent the sums of delta of the pass between,
+    // which this one does after the __syncthreads that follows.
+    auto received = [&](int q, unsigned pass) {
+        if (S == 1) return;
+        const unsigned bar = smem(&bars[q][pass & 1u]), phase = (q == 2 ? pass - 1 : pass) >> 1;
+        const bool ok = wait_for(
+            [&] {
+                unsigned there;
+                asm volatile(
+                    "{\n.reg .pred p;\nmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+                    "selp.u32 %0, 1, 0, p;\n}"
+                    : "=r"(there)
+                    : "r"(bar), "r"(phase & 1u)
+                    : "memory");
+                return bool(__all_sync(0xffffffffu, there != 0u));
+            },
+            8 * kSpinLimit, &st->fail);
+        if (!ok) failed();
+        else if (lane == 0) expect(q, pass);
     };
-    // waits until every cluster has arrived at counter b (`target` arrivals)
-    auto meet = [&](int b, unsigned target) {
+    // waits until every block has added to counter b in this pass
+    auto meet = [&](int b) {
         __syncwarp();
-        if (lane == 0) {
-            if (rank == 0) arrive(&st->bar[b]);
-            if (!wait(&st->bar[b], target)) failed();
-        }
-        __syncwarp();
+        if (lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar[b]) : "memory");
+        const bool ok = wait_for(
+            [&] {
+                unsigned v;
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->bar[b]) : "memory");
+                return bool(__all_sync(0xffffffffu, int(v - ph * unsigned(clusters)) >= 0));
+            },
+            kSpinLimit, &st->fail);
+        if (!ok) failed();
     };
-    // the sum of quantity q over all chunks; one cluster reads its thread
-    // sums directly, ordered by the cluster's own barriers
+    auto put_part = [&](int q, int ch, double v) {
+        const long i = long(2 * q + int(ph & 1u)) * nb + ch;
+        if (counted_sums) __stcg(reinterpret_cast<double*>(A.part) + i, v);
+        else put_slot(A.part + i, v, pass0 + ph);
+    };
+    // the calling warp: quantity q summed over all chunks; `pass`: whose thread
+    // sums.  One warp of each cluster publishes its chunks' sums (of delta,
+    // with S == 1, the warps that own the cells did).
     auto total = [&](int q, unsigned pass) {
-        return single ? warp_chunk_sum<S>(tv(q, 0, pass), min(n, 256), cl) : warp_final_sum(A.part + q * nb, nb);
+        if (single) {
+            received(q, pass);
+            return __shfl_sync(0xffffffffu, warp_chunk_sum(tv(q, 0, pass), min(n, 256)), 0);
+        }
+        if (rank == 0 && (S > 1 || q != 2)) {
+            received(q, pass);
+            int lc = 0;
+            for (int ch = cluster; ch < nb; ch += clusters, ++lc) {
+                const double v = warp_chunk_sum(tv(q, lc, pass), min(n - ch * kChunk, 256));
+                if (lane == 0) put_part(q, ch, v);
+            }
+        }
+        if (counted_sums) meet(q);
+        bool ok = true;
+        const long set = long(2 * q + int(ph & 1u)) * nb;
+        const double v =
+            counted_sums ? warp_final_sum<8>(reinterpret_cast<const double*>(A.part) + set, nb, 0u, &st->fail, &ok)
+                         : warp_final_sum<sums_per_lane(S)>(A.part + set, nb, pass0 + ph, &st->fail, &ok);
+        if (!ok) failed();
+        return v;
     };
-    sync_all();
 
     // ---- r = b - M x, u = D^-1 r ----
     if (mine) {
@@ -329,27 +443,51 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
             chain(0, vals, vals + M, 0);
             chain(1, vals, vals, kNext);
             chain(3, vals + 2 * M, vals + 2 * M, 2 * kNext);
+            bar_sync(kBarMain, M);   // vals + 2 M holds w from now on
         }
+        if (S == 1) bar_arrive(kBarG, M + kWarpsG);
     }
     int k = -1, done = 0, converged = 0;
     double alpha = 0.0;
     while (true) {
-        sync_all();
-        if (sc.fail) break;
         ++ph;
+        Scalars& sc = scalars[ph & 1u];
         if (mine) {
             // ---- w = M u ----
-            if (!single) bar_sync(kBarU, M + 32);
+            if (counted) bar_sync(kBarU, M + 32);
+            const PcgSlot* const u = A.u + long(ph & 1u) * n;
             int lc = 0;
             for (int ch = cluster; ch < nb; ch += clusters, ++lc) {
                 double sd = 0.0;
+                if (Mode != kReg) {
+#pragma unroll
+                    for (int j = 0; j < I; ++j) load_cell(min(cell(ch, j), long(n) - 1), j);
+                }
                 double un[I][6];
+                if constexpr (alone || counted) {
+                    const double* const ud = alone ? vals + M : reinterpret_cast<const double*>(A.u);
 #pragma unroll
-                for (int j = 0; j < I; ++j) {
-                    const long c = min(cell(ch, j), long(n) - 1);
-                    if (Mode != kReg) load_cell(c, j);
+                    for (int j = 0; j < I; ++j) {
+                        const long c = min(cell(ch, j), long(n) - 1);
 #pragma unroll
-                    for (int f = 0; f < 6; ++f) un[j][f] = get_u(nbr[j][f] >= 0 ? nbr[j][f] : c);
+                        for (int f = 0; f < 6; ++f) {
+                            const long i = nbr[j][f] >= 0 ? nbr[j][f] : c;
+                            un[j][f] = alone ? ud[i] : __ldcg(ud + i);
+                        }
+                    }
+                } else {
+                    const bool ok = wait_for(
+                        [&] {
+                            bool all = true;
+#pragma unroll
+                            for (int f = 0; f < 6; ++f) {
+                                un[0][f] = 0.0;
+                                if (nbr[0][f] >= 0) all = get_slot(u + nbr[0][f], pass0 + ph, &un[0][f]) && all;
+                            }
+                            return bool(__all_sync(0xffffffffu, all));
+                        },
+                        kSpinLimit, &st->fail);
+                    if (!ok) failed();
                 }
 #pragma unroll
                 for (int j = 0; j < I; ++j) {
@@ -367,19 +505,17 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
                 bar_sync(kBarMain, M);
                 chain(2, vals + 2 * M, vals + M, 0);
             }
-            if (S > 1) {
-                cl.sync();
-            } else if (single) {
+            if (S == 1 && single) {
                 bar_arrive(kBarW, M + 32);
-            } else {
+            } else if (S == 1) {
                 // a warp per chunk forms its sum
                 bar_sync(kBarMain, M);
                 const int w = tid >> 5, ch = cluster + w * clusters;
                 if (w < slots && ch < nb) {
-                    const double v = warp_chunk_sum<S>(tv(2, w, ph), min(n - ch * kChunk, 256), cl);
-                    if (lane == 0) A.part[2 * nb + ch] = v;
+                    const double v = warp_chunk_sum(tv(2, w, ph), min(n - ch * kChunk, 256));
+                    if (lane == 0) put_part(2, ch, v);
                 }
-                bar_arrive(kBarW, M + 32);
+                if (counted_sums) bar_arrive(kBarW, M + 32);
             }
             // ---- while delta is summed: x += alpha p of the last direction,
             //      p = u + beta p, s = w + beta s (p = u, s = w at the start) ----
@@ -406,64 +542,51 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
                 }
         } else if (role == 2) {
             // D: u of every block, then delta and alpha
-            if (!single) {
-                meet(0, ph * unsigned(clusters));
+            if (counted) {
+                bar_sync(kBarG, M + kWarpsG);
+                if (!single) meet(4);
                 bar_arrive(kBarU, M + 32);
             }
-            if (S == 1) bar_sync(kBarW, M + 32);
-            else cl.sync();
-            if (!single) {
-                if (S > 1) publish(2, A.part + 2 * nb, ph);
-                meet(2, ph * unsigned(clusters));
-            }
+            if (S == 1 && (single || counted_sums)) bar_sync(kBarW, M + 32);
             const double d = total(2, ph);
             bar_sync(kBarT, 64);
-            if (lane == 0) {
-                const double g = sc.g;
-                sc.alpha = k < 0 ? g / d : g / (d - sc.t);
-            }
+            if (lane == 0) sc.alpha = k < 0 ? sc.g / d : sc.g / (d - sc.t);
         } else {
             // G: gamma (and b.b at the start), beta; R: r.r
-            if (S > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-            if (!single) {
-                publish(role, A.part + role * nb, ph - 1);
-                if (k < 0 && role == 0) publish(3, A.part + 3 * nb, 0);
-                meet(1, ph * 2u * unsigned(clusters));
-            }
+            if (S == 1) bar_sync(kBarG, M + kWarpsG);
             const double v = total(role, ph - 1);
             if (role == 0) {
-                const double bb = k < 0 ? total(3, 0) : 0.0;
-                const double be = k < 0 ? 0.0 : v / sc.rz;
-                if (lane == 0) {
-                    sc.beta = be;
-                    if (k < 0) {
-                        sc.bb = bb;
-                        sc.lim = (A.tol * A.tol) * bb;
+                const double be = k < 0 ? 0.0 : v / sc_rz;
+                if (k < 0) {
+                    const double bb = total(3, 0);
+                    if (lane == 0) {
+                        sc_bb = bb;
+                        sc_lim = (A.tol * A.tol) * bb;
                     }
                 }
+                if (lane == 0) sc.beta = be;
                 __syncwarp();
                 bar_arrive(kBarBeta, M + 32);
                 if (lane == 0) {
-                    sc.t = k < 0 ? 0.0 : be * v / sc.alpha;
+                    sc.t = k < 0 ? 0.0 : be * v / scalars[(ph - 1) & 1u].alpha;
                     sc.g = v;
-                    sc.rz = v;
+                    sc_rz = v;
                 }
                 __syncwarp();
                 bar_arrive(kBarT, 64);
             } else if (lane == 0) {
                 sc.rr = v;
             }
-            if (S > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         }
-        __syncthreads();
+        if (__syncthreads_or(bad)) break;
         alpha = sc.alpha;
         if (k < 0 && blockIdx.x == 0 && tid == 0) {
             st->rr0 = sc.rr;
-            st->bb = sc.bb;
-            st->lim = sc.lim;
+            st->bb = sc_bb;
+            st->lim = sc_lim;
         }
         ++k;
-        if (sc.rr <= sc.lim) {
+        if (sc.rr <= sc_lim) {
             done = converged = 1;
             break;
         }
@@ -504,6 +627,7 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
                 chain(0, vals, vals + M, 0);
                 chain(1, vals, vals, kNext);
             }
+            if (S == 1) bar_arrive(kBarG, M + kWarpsG);
         }
     }
     // ---- results ----
@@ -516,19 +640,21 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
     }
     if (tid == 0) {
         if (blockIdx.x == 0) {
-            st->rr = sc.rr;
+            st->rr = scalars[ph & 1u].rr;
             st->k = st->iters = k;
             st->done = done;
             st->converged = converged;
         }
-        // the last block out clears the counters for the next solve
+        // the last block out numbers the passes of the next solve on (with
+        // room for blocks a pass apart when one gave up)
         __threadfence();
         if (atomicAdd(&st->exits, 1u) == gridDim.x - 1) {
-            st->bar[0] = st->bar[1] = st->bar[2] = 0u;
+            st->pass = pass0 + ph + 4;
+            for (unsigned& b : st->bar) b = 0u;
             st->exits = 0u;
         }
     }
-    if (S > 1) cl.sync();
+    if (S > 1) cl.sync();   // no block leaves while another may still send to it
 }
 
 using Kernel = void (*)(PcgArgs);
@@ -564,7 +690,7 @@ void configure(const PcgPlan& p, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* a
 
 cudaError_t prepare(PcgPlan* plan, int sm_count, bool uniform) {
     const int slots = (plan->chunks + plan->clusters - 1) / plan->clusters, per = 256 / plan->split;
-    int doubles = kSums * slots * per;
+    int doubles = plan->split > 1 ? 8 * 256 : kSums * slots * 256;
     if (slots > 1) doubles += slots * kVecs * kChunk;
     else if (plan->split > 1) doubles += 3 * kItems * per;
     else if (plan->alone) doubles += 3 * 256;
@@ -608,21 +734,21 @@ cudaError_t pcg_make_plan(int n, bool uniform, PcgPlan* plan) {
     plan->clusters = (plan->chunks + slots - 1) / slots;
     plan->alone = n <= 256;
     for (int split = plan->alone ? 1 : 8; split >= 1 && !plan->fits; split >>= 1) {
-        if (split > 1 && plan->chunks * split > sm) continue;
+        if (split > 1 && (plan->chunks * split > sm || plan->chunks > 32 * sums_per_lane(split))) continue;
         plan->split = split;
         if ((e = prepare(plan, sm, uniform)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
-cudaError_t launch_pcg_solve(const DMesh& m, const PcgPlan& plan, const double* b, double* x, double* u, double* part,
+cudaError_t launch_pcg_solve(const DMesh& m, const PcgPlan& plan, const double* b, double* x, PcgSlot* slots,
                              PcgState* st, double tol, int maxit, cudaStream_t s) {
     PcgArgs A{};
     A.m = m;
     A.b = b;
     A.x = x;
-    A.u = u;
-    A.part = part;
+    A.u = slots;
+    A.part = slots + 2 * long(plan.cells);
     A.st = st;
     A.tol = tol;
     A.maxit = maxit;

@@ -29,6 +29,7 @@ constexpr long kPartDoubles = 4 * kMaxBlocks + 8;
 constexpr long kStateDoubles = 32;  // holds one pgd::PcgState (rounded up)
 constexpr long kNoallocScratchDoubles = 6 * kMaxCells + kPartDoubles + kStateDoubles;
 static_assert(sizeof(pgd::PcgState) <= kStateDoubles * sizeof(double), "state does not fit");
+static_assert(kMaxCells + 1 + 2 * (2 * kMaxCells + 8 * kMaxBlocks) <= 6 * kMaxCells, "the slots do not fit");
 
 // The scratch: dinv | r | u | p | s | w | partial sums | PCG state.
 static __device__ __align__(256) double g_pcg_scratch[kNoallocScratchDoubles];
@@ -97,7 +98,11 @@ extern "C" picgpu_status picgpu_solve_ldu_noalloc(int n_cells, const double* dia
     if (plan.fits) {
         // the persistent solve (pcg.cu): every problem size on a GPU that
         // holds kMaxBlocks blocks
-        if (pgd::launch_pcg_solve(m, plan, b, x, u, part, st, tol, max_iter, s) != cudaSuccess ||
+        // its slots lie where the vectors of the other path do, behind dinv
+        // (16-byte aligned); cleared, as calls differ in size
+        auto* slots = reinterpret_cast<pgd::PcgSlot*>(scratch + (n + 1) / 2 * 2);
+        if (cudaMemsetAsync(slots, 0, sizeof(pgd::PcgSlot) * pgd::pcg_slots(n_cells), s) != cudaSuccess ||
+            pgd::launch_pcg_solve(m, plan, b, x, slots, st, tol, max_iter, s) != cudaSuccess ||
             cudaGetLastError() != cudaSuccess ||
             cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess || h.fail) {
