@@ -85,6 +85,11 @@ struct DMesh {
     int uniform;             // one geometry class (block mesh of equal cells)
     int lap_uniform;         // every coupled face in direction f has M coefficient lap_coef[f]
     double lap_coef[6];
+    // equal boxes: one geometry class with normals along the axes, weights 1/2
+    // on all coupled faces, one volume; per face the non-zero component of the
+    // area vector, and the volume with its reciprocal
+    int box;
+    double box_area[6], box_vol, box_rvol;
 };
 
 // Per-species particle storage (structure of arrays).

@@ -95,21 +95,23 @@ void launch_charge_update_mixed(const DMesh& m, int vw, const SpeciesValues& sv,
 }
 
 // E per cell for the FP32 move kernel: centre value + the 8 corner (point)
-// values as float4, so a particle's field gather reads one cell block.
-__global__ void corner_E_kernel(DMesh m, const double* __restrict__ E, const double* __restrict__ Ept,
+// values as float4, so a particle's field gather reads one cell block.  From
+// the rounded fields: 27 conversions of a double per cell, at the FP64 rate,
+// took longer than the memory.
+__global__ void corner_E_kernel(DMesh m, const float* __restrict__ E32, const float* __restrict__ Ept32,
                                 float4* __restrict__ Ec4) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n_cells) return;
-    const double* e = E + 3 * size_t(c);
-    Ec4[9 * size_t(c)] = make_float4(float(e[0]), float(e[1]), float(e[2]), 0.f);
+    const float* e = E32 + 3 * size_t(c);
+    Ec4[9 * size_t(c)] = make_float4(e[0], e[1], e[2], 0.f);
     for (int q = 0; q < 8; ++q) {
-        const double* p = Ept + 3 * size_t(m.cell_pt[8 * size_t(c) + q]);
-        Ec4[9 * size_t(c) + 1 + q] = make_float4(float(p[0]), float(p[1]), float(p[2]), 0.f);
+        const float* p = Ept32 + 3 * size_t(m.cell_pt[8 * size_t(c) + q]);
+        Ec4[9 * size_t(c) + 1 + q] = make_float4(p[0], p[1], p[2], 0.f);
     }
 }
 
-void launch_corner_E(const DMesh& m, const double* E, const double* Ept, float4* Ec4, cudaStream_t s) {
-    corner_E_kernel<<<(m.n_cells + 255) / 256, 256, 0, s>>>(m, E, Ept, Ec4);
+void launch_corner_E(const DMesh& m, const float* E32, const float* Ept32, float4* Ec4, cudaStream_t s) {
+    corner_E_kernel<<<(m.n_cells + 255) / 256, 256, 0, s>>>(m, E32, Ept32, Ec4);
 }
 
 // FloatingPotential::preUpdate_Boundary (FloatingPotential.C:89-100)
@@ -435,35 +437,79 @@ __global__ void __launch_bounds__(256) of_residual_kernel(DMesh m, const double*
 }
 
 // ------------------------------------------------------------ E field ----
-__global__ void grad_E_kernel(DMesh m, const double* __restrict__ phi,
-                              const double* __restrict__ grad_bc, double* __restrict__ E) {
+// FP64 issue bounds these kernels (64 cycles per warp instruction), not memory.
+// So on equal boxes the zeros of the area vectors, the weights 1/2 and the
+// divisions by the one volume are left out in a way that keeps every bit: 40
+// instructions per cell instead of 108.  With the rounded copies written where
+// the values are (the FP32 form alone reads them) and the corner blocks copied
+// from those, the field of 64^3 cells takes 93 us a step instead of 128.
+
+// x / d with r = 1 / d rounded to nearest: the quotient corrected twice with
+// the exact remainder is correctly rounded (Markstein 1990; Cornea, Harrison,
+// Tang 2002).  Operands near the ends of the range take the division.
+__device__ __forceinline__ double divide_by(double x, double d, double r) {
+    const unsigned h = unsigned(__double2hiint(x)) & 0x7fffffffu;
+    if (h - 0x10000000u >= 0x60000000u) return (h | unsigned(__double2loint(x))) == 0u ? x : x / d;
+    double q = x * r;
+    q = __fma_rn(__fma_rn(-q, d, x), r, q);
+    return __fma_rn(__fma_rn(-q, d, x), r, q);
+}
+
+// phi on the boundary face f of cell c; false when the face is none.
+__device__ __forceinline__ bool boundary_phi(const DMesh& m, const double* grad_bc, int c, int f, double phic,
+                                             double* pf) {
+    const int bf = m.cell_bface[6 * size_t(c) + f];
+    if (bf < 0) return false;
+    const int pa = m.bf_patch[bf];
+    *pf = pg::face_value(pg::face_rule(c_patchF.kind[pa], c_patchF.phi_bc[pa]), c_patchF.phi[pa], grad_bc[pa],
+                         c_patchF.rlc_k[pa], m.bf_delta[bf], phic);
+    return true;
+}
+
+template <bool Box>
+__global__ void grad_E_kernel(DMesh m, const double* __restrict__ phi, const double* __restrict__ grad_bc,
+                              double* __restrict__ E, float* __restrict__ E32) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n_cells) return;
-    const int cl = m.cell_class[c];
-    double g0 = 0.0, g1 = 0.0, g2 = 0.0;
-    for (int f = 0; f < 6; ++f) {
-        const int nb = m.nbr[6 * size_t(c) + f];
-        double pf;
-        if (nb >= 0) {
-            const double w = m.ip_weight[6 * size_t(c) + f];
-            pf = w * phi[c] + (1.0 - w) * phi[nb];
-        } else {
-            const int bf = m.cell_bface[6 * size_t(c) + f];
-            if (bf < 0) continue;
-            const int pa = m.bf_patch[bf];
-            pf = pg::face_value(pg::face_rule(c_patchF.kind[pa], c_patchF.phi_bc[pa]), c_patchF.phi[pa],
-                                grad_bc[pa], c_patchF.rlc_k[pa], m.bf_delta[bf], phi[c]);
+    double g[3] = {0.0, 0.0, 0.0};
+    const double phic = phi[c];
+    bool finite = true;
+    if (Box) {
+        const double half = 0.5 * phic;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            const int nb = m.nbr[6 * size_t(c) + f];
+            double pf = 0.0;
+            if (nb >= 0) pf = half + 0.5 * phi[nb];
+            else if (!boundary_phi(m, grad_bc, c, f, phic, &pf)) continue;
+            finite = finite && (__double2hiint(pf) & 0x7ff00000) != 0x7ff00000;
+            g[f / 2] = g[f / 2] + pf * m.box_area[f];
         }
-        const double area = m.farea[size_t(cl) * 6 + f];
-        const double* n = m.fnormal + size_t(cl) * 18 + 3 * f;
-        g0 = g0 + pf * (n[0] * area);
-        g1 = g1 + pf * (n[1] * area);
-        g2 = g2 + pf * (n[2] * area);
     }
-    const double V = m.vol[c];
-    E[3 * size_t(c)] = -(g0 / V);
-    E[3 * size_t(c) + 1] = -(g1 / V);
-    E[3 * size_t(c) + 2] = -(g2 / V);
+    if (!Box || !finite) {
+        g[0] = g[1] = g[2] = 0.0;
+        const int cl = m.cell_class[c];
+        for (int f = 0; f < 6; ++f) {
+            const int nb = m.nbr[6 * size_t(c) + f];
+            double pf;
+            if (nb >= 0) {
+                const double w = m.ip_weight[6 * size_t(c) + f];
+                pf = w * phic + (1.0 - w) * phi[nb];
+            } else if (!boundary_phi(m, grad_bc, c, f, phic, &pf)) {
+                continue;
+            }
+            const double area = m.farea[size_t(cl) * 6 + f];
+            const double* n = m.fnormal + size_t(cl) * 18 + 3 * f;
+#pragma unroll
+            for (int a = 0; a < 3; ++a) g[a] = g[a] + pf * (n[a] * area);
+        }
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const double e = -(Box ? divide_by(g[a], m.box_vol, m.box_rvol) : g[a] / m.vol[c]);
+        E[3 * size_t(c) + a] = e;
+        if (E32) E32[3 * size_t(c) + a] = float(e);
+    }
 }
 
 __global__ void boundary_E_kernel(DMesh m, const double* __restrict__ phi,
@@ -485,21 +531,19 @@ __global__ void point_E_kernel(DMesh m, const double* __restrict__ E, const doub
                                double* __restrict__ Ept, float* __restrict__ Ept32) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= m.n_points) return;
-    double e0 = 0.0, e1 = 0.0, e2 = 0.0;
+    double e[3] = {0.0, 0.0, 0.0};
     for (int k = m.pi_start[p]; k < m.pi_start[p + 1]; ++k) {
         const int s = m.pi_src[k];
         const double* src = s >= 0 ? E + 3 * size_t(s) : Eb + 3 * size_t(-s - 1);
         const double w = m.pi_w[k];
-        e0 = e0 + w * src[0];
-        e1 = e1 + w * src[1];
-        e2 = e2 + w * src[2];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) e[a] = e[a] + w * src[a];
     }
-    Ept[3 * size_t(p)] = e0;
-    Ept[3 * size_t(p) + 1] = e1;
-    Ept[3 * size_t(p) + 2] = e2;
-    Ept32[3 * size_t(p)] = float(e0);
-    Ept32[3 * size_t(p) + 1] = float(e1);
-    Ept32[3 * size_t(p) + 2] = float(e2);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        Ept[3 * size_t(p) + a] = e[a];
+        if (Ept32) Ept32[3 * size_t(p) + a] = float(e[a]);
+    }
 }
 
 __global__ void to_float_kernel(const double* __restrict__ a, float* __restrict__ b, long n) {
@@ -628,10 +672,10 @@ void launch_of_residual(const DMesh& m, const double* b, const double* x, double
 
 void launch_efield(const DMesh& m, const double* phi, const double* grad_bc, double* E, double* Eb,
                    double* Ept, float* E32, float* Ept32, cudaStream_t s) {
-    grad_E_kernel<<<blocks(m.n_cells, 256), 256, 0, s>>>(m, phi, grad_bc, E);
+    if (m.box) grad_E_kernel<true><<<blocks(m.n_cells, 256), 256, 0, s>>>(m, phi, grad_bc, E, E32);
+    else grad_E_kernel<false><<<blocks(m.n_cells, 256), 256, 0, s>>>(m, phi, grad_bc, E, E32);
     if (m.n_bfaces > 0) boundary_E_kernel<<<blocks(m.n_bfaces, 256), 256, 0, s>>>(m, phi, grad_bc, E, Eb);
     point_E_kernel<<<blocks(m.n_points, 256), 256, 0, s>>>(m, E, Eb, Ept, Ept32);
-    to_float_kernel<<<blocks(3L * m.n_cells, 256), 256, 0, s>>>(E, E32, 3L * m.n_cells);
 }
 
 void launch_to_float(const double* a, float* b, long n, cudaStream_t s) {

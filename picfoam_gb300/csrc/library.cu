@@ -654,11 +654,14 @@ pgd::MoveParams move_params(picgpu_ctx* c, int s, bool deposit_only) {
 }
 
 picgpu_status zero_accumulators(picgpu_ctx* c) {
-    CK(cudaMemsetAsync(c->cc_data, 0, sizeof(double) * c->m.n_cells, c->stream));
-    CK(cudaMemsetAsync(c->vtx_data, 0, sizeof(double) * c->m.n_points, c->stream));
-    CK(cudaMemsetAsync(c->cc_fix, 0, sizeof(long long) * c->m.n_cells, c->stream));
-    CK(cudaMemsetAsync(c->vtx_fix, 0, sizeof(long long) * c->m.n_points, c->stream));
-    if (c->mixed)
+    // the accumulators of this form and deposit mode
+    if (!c->mixed && c->cfg.deposit_mode == PICGPU_DEPOSIT_FIXED_POINT) {
+        CK(cudaMemsetAsync(c->cc_fix, 0, sizeof(long long) * c->m.n_cells, c->stream));
+        CK(cudaMemsetAsync(c->vtx_fix, 0, sizeof(long long) * c->m.n_points, c->stream));
+    } else if (!c->mixed) {
+        CK(cudaMemsetAsync(c->cc_data, 0, sizeof(double) * c->m.n_cells, c->stream));
+        CK(cudaMemsetAsync(c->vtx_data, 0, sizeof(double) * c->m.n_points, c->stream));
+    } else
         CK(cudaMemsetAsync(c->acc9, 0, sizeof(unsigned long long) * c->cfg.n_species * 9 * size_t(c->m.n_cells),
                            c->stream));
     return PICGPU_OK;
@@ -708,10 +711,11 @@ picgpu_status charge_update(picgpu_ctx* c) {
 
 picgpu_status efield(picgpu_ctx* c) {
     PhaseScope ps(c, PICGPU_PHASE_EFIELD);
-    pgd::launch_efield(c->dm, c->phi, c->grad_bc, c->E, c->Eb, c->Ept, c->E32, c->Ept32, c->stream);
-    c->launches += c->dm.n_bfaces > 0 ? 4 : 3;
+    pgd::launch_efield(c->dm, c->phi, c->grad_bc, c->E, c->Eb, c->Ept, c->mixed ? c->E32 : nullptr,
+                       c->mixed ? c->Ept32 : nullptr, c->stream);
+    c->launches += c->dm.n_bfaces > 0 ? 3 : 2;
     if (c->Ec4) {
-        pgd::launch_corner_E(c->dm, c->E, c->Ept, c->Ec4, c->stream);
+        pgd::launch_corner_E(c->dm, c->E32, c->Ept32, c->Ec4, c->stream);
         c->launches++;
     }
     CK(cudaGetLastError());
@@ -728,7 +732,7 @@ picgpu_status set_applied_field(picgpu_ctx* c) {
     pgd::launch_to_float(c->Ept, c->Ept32, long(ep.size()), c->stream);
     c->launches += 2;
     if (c->Ec4) {
-        pgd::launch_corner_E(c->dm, c->E, c->Ept, c->Ec4, c->stream);
+        pgd::launch_corner_E(c->dm, c->E32, c->Ept32, c->Ec4, c->stream);
         c->launches++;
     }
     CK(cudaStreamSynchronize(c->stream));
@@ -1920,6 +1924,20 @@ static picgpu_status create_with_mesh(picgpu_ctx* c, const picgpu_config* cfg) {
             else if (Moff[k] != d.lap_coef[f]) d.lap_uniform = 0;
         }
     }
+    // equal boxes: grad_E then skips the zeros of the area vectors
+    d.box = d.uniform;
+    for (int f = 0; f < 6; ++f) {
+        for (int a = 0; a < 3 && d.box; ++a)
+            if (a != f / 2 && m.cls_fnormal[3 * f + a] != 0.0) d.box = 0;
+        d.box_area[f] = d.box ? m.cls_fnormal[3 * f + f / 2] * m.cls_farea[f] : 0.0;
+    }
+    d.box_vol = m.vol[0];
+    d.box_rvol = 1.0 / m.vol[0];
+    for (size_t k = 0; k < m.ip_weight.size() && d.box; ++k)
+        if (m.nbr[k] >= 0 && m.ip_weight[k] != 0.5) d.box = 0;
+    for (size_t k = 0; k < m.vol.size() && d.box; ++k)
+        if (m.vol[k] != d.box_vol) d.box = 0;
+    if (!(d.box_vol > 0x1p-200 && d.box_vol < 0x1p200)) d.box = 0;
 #undef UP
     (void)ip; (void)dp; (void)fp;
 
@@ -2912,7 +2930,7 @@ picgpu_status picgpu_set_field(picgpu_ctx* c, int which, const double* in, size_
     pgd::launch_to_float(c->Ept, c->Ept32, 3L * c->m.n_points, c->stream);
     c->launches += 2;
     if (c->Ec4) {
-        pgd::launch_corner_E(c->dm, c->E, c->Ept, c->Ec4, c->stream);
+        pgd::launch_corner_E(c->dm, c->E32, c->Ept32, c->Ec4, c->stream);
         c->launches++;
     }
     CK(cudaStreamSynchronize(c->stream));
@@ -3020,7 +3038,7 @@ picgpu_status picgpu_ensemble_set_efield(picgpu_ctx* c, const double* E) {
     pgd::launch_to_float(c->Ept, c->Ept32, long(ep.size()), c->stream);
     c->launches += 2;
     if (c->Ec4) {
-        pgd::launch_corner_E(c->dm, c->E, c->Ept, c->Ec4, c->stream);
+        pgd::launch_corner_E(c->dm, c->E32, c->Ept32, c->Ec4, c->stream);
         c->launches++;
     }
     CK(cudaStreamSynchronize(c->stream));
