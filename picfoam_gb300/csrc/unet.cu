@@ -184,26 +184,36 @@ __global__ void relu_mask_kernel(long n, const float* __restrict__ gr, const __n
 // Splits the gradient of a concatenated decoder input [up(coarse), skip]:
 // g_skip[v][c] += g_cat[v][C1 + c]; g_coarse[vc][c] = sum over the 8 fine
 // children of g_cat[child][c].
-__global__ void split_cat_kernel(ConvGrid g, int C1, int C2, const float* __restrict__ gcat,
-                                 float* __restrict__ gskip, float* __restrict__ gcoarse) {
+// One thread per value, the channels of a voxel together: a thread per coarse
+// voxel, with 16 blocks on the smaller of two grids and neighbours a voxel's
+// channels apart, took 297 us of the 2255 of a 64 x 64 x 32 network's gradient
+// (1990 now).
+template <int C1, int C2>
+__global__ void split_cat_kernel(ConvGrid g, const float* __restrict__ gcat, float* __restrict__ gskip,
+                                 float* __restrict__ gcoarse) {
+    constexpr int C = C1 + C2;
     const ConvGrid h{g.X / 2, g.Y / 2, g.Z / 2};
     const long Vc = long(h.X) * h.Y * h.Z;
-    const long i = long(blockIdx.x) * blockDim.x + threadIdx.x;
+    const long t = long(blockIdx.x) * blockDim.x + threadIdx.x;
+    const bool sum = t < Vc * C1;
+    const long u = t - Vc * C1;
+    const long i = sum ? t / C1 : u / (8 * C2);
     if (i >= Vc) return;
-    const Coord c = coord(i, h);
-    const int C = C1 + C2;
-    for (int ch = 0; ch < C1; ++ch) {
+    const int v = int(i), x = v % h.X, yz = v / h.X, y = yz % h.Y, z = yz / h.Y;
+    auto fine = [&](int k) {
+        return (long(2 * z + (k >> 2)) * g.Y + 2 * y + ((k >> 1) & 1)) * g.X + 2 * x + (k & 1);
+    };
+    if (sum) {
+        const int ch = int(t % C1);
         float s = 0.f;
-        for (int k = 0; k < 8; ++k) {
-            const long vf = (long(2 * c.z + (k >> 2)) * g.Y + 2 * c.y + ((k >> 1) & 1)) * g.X + 2 * c.x + (k & 1);
-            s += gcat[vf * C + ch];
-        }
-        gcoarse[i * C1 + ch] = s;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += gcat[fine(k) * C + ch];
+        gcoarse[t] = s;
+        return;
     }
-    for (int k = 0; k < 8; ++k) {
-        const long vf = (long(2 * c.z + (k >> 2)) * g.Y + 2 * c.y + ((k >> 1) & 1)) * g.X + 2 * c.x + (k & 1);
-        for (int ch = 0; ch < C2; ++ch) gskip[vf * C2 + ch] += gcat[vf * C + C1 + ch];
-    }
+    const int ch = int(u % C2);
+    const long vf = fine(int(u / C2 % 8));
+    gskip[vf * C2 + ch] += gcat[vf * C + C1 + ch];
 }
 
 // g_fine[v][c] += g_coarse[parent(v)][c] / 8  (average pooling backward).
@@ -505,7 +515,7 @@ cudaError_t UNet::backward(cudaStream_t s) {
     if ((e = dw(8, g1_, hb_, {a_[8], 32, 1}, {a_[2], 16, 0}, nullptr, s))) return e;
     if ((e = tc_dx(8, g1_, gA_, s))) return e;  // g_cat [V1][48]
     zero(gskip1_, 16 * size_t(V1_), s);
-    split_cat_kernel<<<nblk(V2), 256, 0, s>>>(g1_, 32, 16, gA_, gskip1_, gC_);  // g_a8 -> gC_ [V2][32]
+    split_cat_kernel<32, 16><<<nblk(V2 * (32 + 8 * 16)), 256, 0, s>>>(g1_, gA_, gskip1_, gC_);  // g_a8 -> gC_ [V2][32]
     // a8 = relu(d2b(a7))
     mask(gC_, a_[8], 32 * V2, s);
     if ((e = dw(7, g2_, hb_, {a_[7], 32, 0}, none, nullptr, s))) return e;
@@ -515,7 +525,7 @@ cudaError_t UNet::backward(cudaStream_t s) {
     if ((e = dw(6, g2_, hb_, {a_[6], 64, 1}, {a_[4], 32, 0}, nullptr, s))) return e;
     if ((e = tc_dx(6, g2_, gA_, s))) return e;  // g_cat [V2][96]
     zero(gskip2_, 32 * size_t(V2), s);
-    split_cat_kernel<<<nblk(V3), 256, 0, s>>>(g2_, 64, 32, gA_, gskip2_, gC_);  // g_a6 -> gC_ [V3][64]
+    split_cat_kernel<64, 32><<<nblk(V3 * (64 + 8 * 32)), 256, 0, s>>>(g2_, gA_, gskip2_, gC_);  // g_a6 -> gC_ [V3][64]
     // a6 = relu(c3b(a5))
     mask(gC_, a_[6], 64 * V3, s);
     if ((e = dw(5, g3_, hb_, {a_[5], 64, 0}, none, nullptr, s))) return e;
