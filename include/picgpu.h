@@ -747,6 +747,11 @@ picgpu_status picgpu_solve_ldu_noalloc(int n_cells, const double* diag, const do
                                        double tol, int max_iter, int* iterations,
                                        double* residual, void* stream);
 
+/* For tests: how many blocks per cluster the persistent Poisson solve of this
+ * context is told to find.  Where that is not what it finds, it does nothing,
+ * and the two-kernel iteration solves from then on. */
+picgpu_status picgpu_test_pcg_ranks(picgpu_ctx* ctx, int ranks);
+
 #ifdef __cplusplus
 }
 #endif

@@ -20,17 +20,21 @@ struct PcgState {
     int done, iters, converged, k;
     unsigned int ticket;
     // persistent solve (pcg.cu): number of its last pass, arrivals, blocks gone,
-    // a wait ran out
+    // why it gave up (kPcgWait, kPcgShape; 0: it did not)
     unsigned int pass, bar[5], exits;
     int fail;
     double rr0;   // r.r of the start guess
 };
+
+constexpr int kPcgWait = 1;    // a wait ran out
+constexpr int kPcgShape = 2;   // clusters of another size than the plan's: nothing was done
 
 // Launch shape of the persistent solve (pcg.cu) for one problem size.
 struct PcgPlan {
     int cells = 0;
     int chunks = 0;     // kChunk cells each
     int split = 1;      // blocks (one cluster) per chunk
+    int ranks = 1;      // what the kernel is told of it
     int clusters = 0;
     int smem = 0;
     bool alone = false; // one block, at most 256 cells

@@ -739,28 +739,72 @@ picgpu_status set_applied_field(picgpu_ctx* c) {
     return PICGPU_OK;
 }
 
+// Jacobi PCG as a CUDA graph of kGraphIters iterations (2 kernels each):
+// iterations after convergence return at once, so the iteration count stays
+// exact, and the host checks the done flag after each replay.
+picgpu_status solve_streamed(picgpu_ctx* c, double tol, int maxit) {
+    if (!c->pcg_graph) {
+        cudaGraph_t g;
+        CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+        for (int j = 0; j < kGraphIters; ++j)
+            pgd::launch_pcg_iteration(c->dm, c->phi, c->r, c->z, c->q, c->p[0], c->p[1], c->part, c->st, maxit,
+                                      c->stream);
+        CK(cudaStreamEndCapture(c->stream, &g));
+        CK(cudaGraphInstantiate(&c->pcg_graph, g, 0));
+        CK(cudaGraphDestroy(g));
+    }
+    pgd::launch_pcg_init(c->dm, c->b, c->phi, c->r, c->z, c->q, c->part, c->st, tol, c->stream);
+    c->launches += 2;
+    CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    c->pcg_r0 = c->st_host->bb > 0 ? std::sqrt(c->st_host->rr / c->st_host->bb) : 0.0;
+    int launched = 0;
+    while (!c->st_host->done && launched < maxit) {
+        CK(cudaGraphLaunch(c->pcg_graph, c->stream));
+        launched += kGraphIters;
+        c->launches += 2 * kGraphIters;
+        CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
+        CK(cudaStreamSynchronize(c->stream));
+    }
+    return PICGPU_OK;
+}
+
+// The state and the exchanged values after a persistent solve that gave up.
+picgpu_status reset_persistent(picgpu_ctx* c) {
+    CK(cudaMemset(c->st, 0, sizeof(pgd::PcgState)));
+    CK(cudaMemset(c->pcg_slots, 0, sizeof(pgd::PcgSlot) * pgd::pcg_slots(c->m.n_cells)));
+    return PICGPU_OK;
+}
+
+// The Jacobi PCG: one persistent launch where every block fits the chip at
+// once (pcg.cu), else the two-kernel iteration; the state is copied to the host
+// behind it.  A persistent solve that gave up says so in st_host->fail.
+picgpu_status solve_jacobi(picgpu_ctx* c, double tol, int maxit, bool learned) {
+    picgpu_status s;
+    if (c->pcg_plan.fits) {
+        CK(pgd::launch_pcg_solve(c->dm, c->pcg_plan, c->b, c->phi, c->pcg_slots, c->st, tol, maxit, c->stream));
+        c->launches += 1;
+    } else if ((s = solve_streamed(c, tol, maxit))) {
+        return s;
+    }
+    pgd::launch_of_residual(c->dm, c->b, c->phi, c->part, c->st, c->stream);
+    c->launches += 2;
+    CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
+    if (learned && c->ws) {
+        CK(cudaStreamSynchronize(c->stream));
+        if (c->st_host->fail == pgd::kPcgShape) return PICGPU_OK;   // solved again, by the other path
+        CK(c->ws->after(c->dm, c->phi, c->st_host->iters, c->stream));
+    }
+    return PICGPU_OK;
+}
+
 // Poisson PCG from the current phi; fills stats.
 picgpu_status poisson(picgpu_ctx* c, picgpu_step_stats* stats, bool learned = false) {
-    const int n = c->m.n_cells;
     const double tol = c->cfg.pcg_tol > 0 ? c->cfg.pcg_tol : 1e-10;
     const int maxit = c->cfg.pcg_max_iter > 0 ? c->cfg.pcg_max_iter : 10000;
+    picgpu_status s;
     {
         PhaseScope ps(c, PICGPU_PHASE_POISSON);
-        // Jacobi PCG: one persistent launch where every block fits the chip
-        // at once (pcg.cu); on larger meshes a CUDA graph of kGraphIters
-        // iterations (2 kernels each), where iterations after convergence
-        // return at once, so the iteration count stays exact, and the host
-        // checks the done flag after each replay.
-        if (!c->pcg_graph && !c->mg && !c->pcg_plan.fits) {
-            cudaGraph_t g;
-            CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-            for (int j = 0; j < kGraphIters; ++j)
-                pgd::launch_pcg_iteration(c->dm, c->phi, c->r, c->z, c->q, c->p[0], c->p[1], c->part, c->st, maxit,
-                                          c->stream);
-            CK(cudaStreamEndCapture(c->stream, &g));
-            CK(cudaGraphInstantiate(&c->pcg_graph, g, 0));
-            CK(cudaGraphDestroy(g));
-        }
         pgd::launch_rhs(c->dm, c->rho, c->grad_bc, c->b, !c->m.has_dirichlet, c->part, c->st, c->stream);
         if (learned && c->ws) {
             CK(c->ws->before(c->dm, c->b, c->phi, c->stream));
@@ -785,48 +829,29 @@ picgpu_status poisson(picgpu_ctx* c, picgpu_step_stats* stats, bool learned = fa
             c->st_host->rr = rr;
             c->st_host->bb = bb;
             c->st_host->converged = conv ? 1 : 0;
-        } else if (c->pcg_plan.fits) {
-            CK(pgd::launch_pcg_solve(c->dm, c->pcg_plan, c->b, c->phi, c->pcg_slots, c->st, tol, maxit, c->stream));
-            pgd::launch_of_residual(c->dm, c->b, c->phi, c->part, c->st, c->stream);
-            c->launches += 3;
-            CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
-            if (learned && c->ws) {
-                CK(cudaStreamSynchronize(c->stream));
-                CK(c->ws->after(c->dm, c->phi, c->st_host->iters, c->stream));
-            }
-        } else {
-            pgd::launch_pcg_init(c->dm, c->b, c->phi, c->r, c->z, c->q, c->part, c->st, tol, c->stream);
-            c->launches += 2;
-            CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
-            CK(cudaStreamSynchronize(c->stream));
-            c->pcg_r0 = c->st_host->bb > 0 ? std::sqrt(c->st_host->rr / c->st_host->bb) : 0.0;
-            int launched = 0;
-            while (!c->st_host->done && launched < maxit) {
-                CK(cudaGraphLaunch(c->pcg_graph, c->stream));
-                launched += kGraphIters;
-                c->launches += 2 * kGraphIters;
-                CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
-                CK(cudaStreamSynchronize(c->stream));
-            }
-            pgd::launch_of_residual(c->dm, c->b, c->phi, c->part, c->st, c->stream);
-            c->launches += 2;
-            if (learned && c->ws) CK(c->ws->after(c->dm, c->phi, c->st_host->iters, c->stream));
-            CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
+        } else if ((s = solve_jacobi(c, tol, maxit, learned))) {
+            return s;
         }
     }
-    picgpu_status s = efield(c);
-    if (s) return s;
+    if ((s = efield(c))) return s;
     CK(cudaStreamSynchronize(c->stream));
-    (void)n;
-    const pgd::PcgState& S = *c->st_host;
-    if (!c->mg && c->pcg_plan.fits) {
-        if (S.fail) {
-            CK(cudaMemset(c->st, 0, sizeof(pgd::PcgState)));
-            CK(cudaMemset(c->pcg_slots, 0, sizeof(pgd::PcgSlot) * pgd::pcg_slots(c->m.n_cells)));
+    if (!c->mg && c->pcg_plan.fits && c->st_host->fail) {
+        const int why = c->st_host->fail;
+        if ((s = reset_persistent(c))) return s;
+        if (why != pgd::kPcgShape)
             return bad(c, PICGPU_CUDA_ERROR, "Poisson PCG: a block of the solver kernel waited too long for the others");
+        // clusters are not as planned here: the two-kernel iteration from now
+        // on, on the system that the persistent solve left untouched
+        c->pcg_plan.fits = false;
+        {
+            PhaseScope ps(c, PICGPU_PHASE_POISSON);
+            if ((s = solve_jacobi(c, tol, maxit, learned))) return s;
         }
-        c->pcg_r0 = S.bb > 0 ? std::sqrt(S.rr0 / S.bb) : 0.0;
+        if ((s = efield(c))) return s;
+        CK(cudaStreamSynchronize(c->stream));
     }
+    const pgd::PcgState& S = *c->st_host;
+    if (!c->mg && c->pcg_plan.fits) c->pcg_r0 = S.bb > 0 ? std::sqrt(S.rr0 / S.bb) : 0.0;
     if (stats) {
         stats->pcg_iterations = S.iters;
         stats->pcg_iterations_total += S.iters;
@@ -2994,6 +3019,12 @@ int64_t picgpu_kernel_launches(const picgpu_ctx* c) { return c ? c->launches : 0
 picgpu_status picgpu_synchronize(picgpu_ctx* c) {
     if (!c) return PICGPU_INVALID_ARG;
     CK(cudaStreamSynchronize(c->stream));
+    return PICGPU_OK;
+}
+
+picgpu_status picgpu_test_pcg_ranks(picgpu_ctx* c, int ranks) {
+    if (!c) return PICGPU_INVALID_ARG;
+    c->pcg_plan.ranks = ranks;
     return PICGPU_OK;
 }
 

@@ -83,6 +83,7 @@ struct PcgArgs {
     double tol;
     int maxit;
     int chunks;
+    int ranks;          // blocks per cluster that the plan counts on
 };
 
 constexpr int threads_of(int I, int S) { return (I == 1 && S > 1 ? kChunk / S : 256) + kScalarThreads; }
@@ -233,12 +234,19 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 // whole chunks, 1 when it shares one or is alone with at most 256 cells.
 // Threads [0, M) own the block's cells; warps G, R and D the scalars.
 template <bool Uniform, int Mode, int I, int S>
-__global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
+__device__ __forceinline__ void pcg_body(const PcgArgs& A) {
     extern __shared__ double dyn[];   // sums; then kSmem: the vectors, I = 1: r, u, w of the block
     __shared__ Scalars scalars[2];    // in turn: a warp may still read one pass's while the next one's are written
     __shared__ double sc_rz, sc_bb, sc_lim;
     __shared__ __align__(8) u64 bars[4][2];   // S > 1: bytes received, per quantity, odd and even passes
     const cg::cluster_group cl = cg::this_cluster();
+    // Every address of a peer below counts on S blocks per cluster.  A launch
+    // that formed other ones (a tool between this library and the driver that
+    // repeats the launch without its cluster) is given back untouched.
+    if (S > 1 && (cl.num_blocks() != unsigned(S) || A.ranks != S)) {
+        if (threadIdx.x == 0) atomicMax(&A.st->fail, kPcgShape);
+        return;
+    }
     constexpr bool alone = I == 1 && S == 1;   // one block, at most 256 cells
     // whole chunks per block: u as it is, an arrival counter instead of slots
     constexpr bool counted = I > 1;
@@ -334,7 +342,7 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
     };
     auto failed = [&]() {
         bad = true;
-        if (lane == 0) atomicMax(&st->fail, 1);
+        if (lane == 0) atomicMax(&st->fail, kPcgWait);
     };
     // S > 1, the calling warp: the pass's sums of quantity q are there.  Its
     // barrier is armed again at once, for two passes later: no block sends
@@ -657,18 +665,29 @@ __global__ void __launch_bounds__(threads_of(I, S)) pcg_kernel(PcgArgs A) {
     if (S > 1) cl.sync();   // no block leaves while another may still send to it
 }
 
+template <bool Uniform, int Mode, int I>
+__global__ void __launch_bounds__(threads_of(I, 1)) pcg_kernel(PcgArgs A) {
+    pcg_body<Uniform, Mode, I, 1>(A);
+}
+
+// The cluster's size belongs to the kernel, so no launch can be without it.
+template <bool Uniform, int S>
+__global__ void __cluster_dims__(S, 1, 1) __launch_bounds__(threads_of(1, S)) pcg_cluster_kernel(PcgArgs A) {
+    pcg_body<Uniform, kReg, 1, S>(A);
+}
+
 using Kernel = void (*)(PcgArgs);
 
 template <bool Uniform>
 Kernel kernel_of(const PcgPlan& p) {
     switch (p.split) {
-        case 8: return pcg_kernel<Uniform, kReg, 1, 8>;
-        case 4: return pcg_kernel<Uniform, kReg, 1, 4>;
-        case 2: return pcg_kernel<Uniform, kReg, 1, 2>;
+        case 8: return pcg_cluster_kernel<Uniform, 8>;
+        case 4: return pcg_cluster_kernel<Uniform, 4>;
+        case 2: return pcg_cluster_kernel<Uniform, 2>;
         default: break;
     }
-    if (p.alone) return pcg_kernel<Uniform, kReg, 1, 1>;
-    return p.clusters >= p.chunks ? pcg_kernel<Uniform, kReg, kItems, 1> : pcg_kernel<Uniform, kSmem, kItems, 1>;
+    if (p.alone) return pcg_kernel<Uniform, kReg, 1>;
+    return p.clusters >= p.chunks ? pcg_kernel<Uniform, kReg, kItems> : pcg_kernel<Uniform, kSmem, kItems>;
 }
 
 Kernel kernel_of(const PcgPlan& p, bool uniform) { return uniform ? kernel_of<true>(p) : kernel_of<false>(p); }
@@ -682,10 +701,7 @@ void configure(const PcgPlan& p, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* a
     cfg->attrs = attr;
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = p.split;
-    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
-    cfg->numAttrs = p.split > 1 ? 2 : 1;
+    cfg->numAttrs = 1;
 }
 
 cudaError_t prepare(PcgPlan* plan, int sm_count, bool uniform) {
@@ -699,7 +715,7 @@ cudaError_t prepare(PcgPlan* plan, int sm_count, bool uniform) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, plan->smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     configure(*plan, &cfg, attr);
     int fit = 0;
     if (plan->split > 1) {
@@ -735,7 +751,7 @@ cudaError_t pcg_make_plan(int n, bool uniform, PcgPlan* plan) {
     plan->alone = n <= 256;
     for (int split = plan->alone ? 1 : 8; split >= 1 && !plan->fits; split >>= 1) {
         if (split > 1 && (plan->chunks * split > sm || plan->chunks > 32 * sums_per_lane(split))) continue;
-        plan->split = split;
+        plan->split = plan->ranks = split;
         if ((e = prepare(plan, sm, uniform)) != cudaSuccess) return e;
     }
     return cudaSuccess;
@@ -753,8 +769,9 @@ cudaError_t launch_pcg_solve(const DMesh& m, const PcgPlan& plan, const double* 
     A.tol = tol;
     A.maxit = maxit;
     A.chunks = plan.chunks;
+    A.ranks = plan.ranks;
     cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     configure(plan, &cfg, attr);
     cfg.stream = s;
     return cudaLaunchKernelEx(&cfg, kernel_of(plan, m.lap_uniform != 0), A);

@@ -105,13 +105,17 @@ extern "C" picgpu_status picgpu_solve_ldu_noalloc(int n_cells, const double* dia
             pgd::launch_pcg_solve(m, plan, b, x, slots, st, tol, max_iter, s) != cudaSuccess ||
             cudaGetLastError() != cudaSuccess ||
             cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess || h.fail) {
+            cudaStreamSynchronize(s) != cudaSuccess || h.fail == pgd::kPcgWait) {
             cudaGetLastError();
             return PICGPU_CUDA_ERROR;
         }
-        if (iterations) *iterations = h.iters;
-        if (residual) *residual = h.bb > 0 ? std::sqrt(h.rr / h.bb) : 0.0;
-        return h.converged ? PICGPU_OK : PICGPU_PCG_NOT_CONVERGED;
+        if (h.fail != pgd::kPcgShape) {
+            if (iterations) *iterations = h.iters;
+            if (residual) *residual = h.bb > 0 ? std::sqrt(h.rr / h.bb) : 0.0;
+            return h.converged ? PICGPU_OK : PICGPU_PCG_NOT_CONVERGED;
+        }
+        // clusters of another size than planned: x is as it was
+        if (cudaMemsetAsync(st, 0, sizeof(pgd::PcgState), s) != cudaSuccess) return PICGPU_CUDA_ERROR;
     }
     pgd::launch_pcg_init(m, b, x, r, u, w, part, st, tol, s);
     // a launch error of the set-up kernels must not pass for convergence when

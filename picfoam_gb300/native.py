@@ -98,6 +98,8 @@ def load():
     lib.picgpu_solve_ldu_noalloc.restype = i
     lib.picgpu_solve_ldu_noalloc.argtypes = [i, P, P, P, P, P, C.c_double, i, C.POINTER(C.c_int),
                                              F64P, P]
+    lib.picgpu_test_pcg_ranks.restype = i
+    lib.picgpu_test_pcg_ranks.argtypes = [P, i]
     U16P = C.POINTER(C.c_uint16)
     F32P = C.POINTER(C.c_float)
     lib.picgpu_test_conv3d.restype = i
