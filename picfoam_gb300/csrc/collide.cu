@@ -46,13 +46,13 @@ __device__ __forceinline__ double eps0c() { return 1.0 / (kMu0c * kC * kC); }
 // it, publishes its sum and walks back over its predecessors' published sums
 // until it meets one whose prefix is known (decoupled look-back; Merrill &
 // Garland 2016).  A state word holds a status and up to 62 bits of sums, so it
-// is read whole.  The last block out clears the state for the next scan.  It
-// took three launches (tile sums, their scan, the tiles' scans), 15 of a swarm
+// is read whole.  A block whose predecessors' sums do not come within its polls
+// adds up the items before its tile itself, so a scan always succeeds.  The last
+// block out clears the state for the next scan.  It took three launches (tile sums, their scan, the tiles' scans), 15 of a swarm
 // step's 33; with these, the two secondaries' append in one launch and the
 // counters per block, a swarm pass of 10^7 electrons went from 7.50 to 6.06 ms
 // and one of 64 cases from 17.1 to 15.1 ms.
 constexpr int kScanThreads = 1024, kScanItems = 4, kScanTile = kScanThreads * kScanItems;
-constexpr unsigned kScanSpin = 1u << 21;   // polls of one predecessor
 constexpr u64 kScanSum = 1ull << 62, kScanPrefix = 2ull << 62, kScanValue = kScanSum - 1;
 
 struct ScanState {
@@ -73,8 +73,10 @@ __device__ __forceinline__ int scan_item(int j) {
 }
 
 // v[j] of the tile's items -> their exclusive prefix over all tiles; returns
-// the prefix behind the tile.  A wait that runs out raises *err.
-__device__ __forceinline__ u64 scan_tile(ScanState* st, int tile, u64 (&v)[kScanItems], int* err) {
+// the prefix behind the tile.  item(i): item i of an earlier tile; polls: how
+// often the sums of 32 predecessors are looked for.
+template <class Item>
+__device__ __forceinline__ u64 scan_tile(ScanState* st, int tile, u64 (&v)[kScanItems], unsigned polls, Item item) {
     __shared__ u64 ws[32];
     __shared__ u64 before;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -109,12 +111,16 @@ __device__ __forceinline__ u64 scan_tile(ScanState* st, int tile, u64 (&v)[kScan
         for (int base = tile - 1; base >= 0; base -= 32) {
             const int p = base - lane;
             u64 w = kScanPrefix;
-            unsigned tries = 0;
-            do {
+            bool there = false;
+            for (unsigned tries = 0; tries < polls && !there; ++tries) {
                 if (p >= 0) w = state[p];
-            } while (!__all_sync(0xffffffffu, w >= kScanSum) && ++tries < kScanSpin);
-            if (tries == kScanSpin) {
-                if (lane == 0) atomicExch(err, 1);
+                there = __all_sync(0xffffffffu, w >= kScanSum);
+            }
+            if (!there) {
+                prefix = 0;
+                for (long i = lane; i < long(tile) * kScanTile; i += 32) prefix += item(i);
+#pragma unroll
+                for (int off = 16; off >= 1; off >>= 1) prefix += __shfl_xor_sync(0xffffffffu, prefix, off);
                 break;
             }
             const unsigned known = __ballot_sync(0xffffffffu, w >= kScanPrefix);
@@ -155,7 +161,7 @@ __device__ __forceinline__ bool scan_finish(ScanState* st) {
 
 __global__ void __launch_bounds__(kScanThreads) exclusive_scan_kernel(const int* __restrict__ in, long n,
                                                                       int* __restrict__ out, ScanState* st,
-                                                                      int* err) {
+                                                                      unsigned polls) {
     const int tile = scan_ticket(st);
     const long base = long(tile) * kScanTile;
     u64 v[kScanItems];
@@ -164,7 +170,7 @@ __global__ void __launch_bounds__(kScanThreads) exclusive_scan_kernel(const int*
         const long i = base + scan_item(j);
         v[j] = i < n ? u64(unsigned(in[i])) : 0;
     }
-    const u64 behind = scan_tile(st, tile, v, err);
+    const u64 behind = scan_tile(st, tile, v, polls, [&](long i) { return u64(unsigned(in[i])); });
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j) {
         const long i = base + scan_item(j);
@@ -180,9 +186,9 @@ unsigned scan_blocks(long n) { return unsigned((n + kScanTile - 1) / kScanTile);
 long scan_ints(long n) { return 2 + 2 * long(scan_blocks(n)) + 2; }
 
 // out[0..n) exclusive prefix of in (counts >= 0), out[n] = total
-void exclusive_scan(const int* in, int* out, long n, int* state, int* err, cudaStream_t s, int64_t* launches) {
+void exclusive_scan(const int* in, int* out, long n, int* state, unsigned polls, cudaStream_t s, int64_t* launches) {
     exclusive_scan_kernel<<<scan_blocks(n), kScanThreads, 0, s>>>(in, n, out, reinterpret_cast<ScanState*>(state),
-                                                                  err);
+                                                                  polls);
     *launches += 1;
 }
 
@@ -795,20 +801,23 @@ __global__ void __launch_bounds__(kScanThreads) append_secondaries_kernel(const 
                                                                           const Secondary* __restrict__ stage, long n,
                                                                           const int* used_dev, int mask, AppendTarget e,
                                                                           AppendTarget ion, u64* added,
-                                                                          ScanState* st, int* overflow) {
+                                                                          ScanState* st, unsigned polls,
+                                                                          int* overflow) {
     const long used = used_dev ? min(long(*used_dev), n) : n;
     const long base[2] = {e.n_dev ? *e.n_dev : e.base, ion.n_dev ? *ion.n_dev : ion.base};
     const int tile = scan_ticket(st);
     const long first = long(tile) * kScanTile;
     int f[kScanItems];
     u64 v[kScanItems];
+    auto both = [](int flag) { return u64(flag & 1) | u64((flag >> 1) & 1) << 31; };
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j) {
         const long i = first + scan_item(j);
         f[j] = i < used ? flags[i] & mask : 0;
-        v[j] = u64(f[j] & 1) | u64((f[j] >> 1) & 1) << 31;
+        v[j] = both(f[j]);
     }
-    const u64 behind = scan_tile(st, tile, v, overflow);
+    const u64 behind =
+        scan_tile(st, tile, v, polls, [&](long i) { return i < used ? both(flags[i] & mask) : u64(0); });
 #pragma unroll
     for (int j = 0; j < kScanItems; ++j) {
         if (!f[j]) continue;
@@ -2538,7 +2547,7 @@ int occupancy(CollideState& st, const CollideArgs& a, int s, std::string* msg, i
         count_cells_kernel<<<grid_of(n, 256), 256, 0, a.stream>>>(a.sp[s].tet, int(n), cnt);
         *launches += 1;
     }
-    exclusive_scan(cnt, start, nc, st.scan_tmp, st.overflow, a.stream, launches);
+    exclusive_scan(cnt, start, nc, st.scan_tmp, st.scan_polls, a.stream, launches);
     if (n > 0) {
         scatter_cells_kernel<<<grid_of(n, 256), 256, 0, a.stream>>>(a.sp[s].tet, int(n), start, st.cell_cursor,
                                                                     st.idx[s]);
@@ -2575,12 +2584,11 @@ int sort_species(CollideState& st, const DMesh& m, int s, const DSpecies& src, c
     if (!st.cell_start) {
         if (dmalloc(&st.cell_start, size_t(PICGPU_MAX_SPECIES) * (nc + 1)) ||
             dmalloc(&st.cell_count, size_t(PICGPU_MAX_SPECIES) * (nc + 1)) || dmalloc(&st.cell_cursor, nc + 1) ||
-            dmalloc(&st.counts, kCollideCounts + 2) || dmalloc(&st.scan_tmp, scan_ints(nc)) || dmalloc(&st.overflow, 1)) {
+            dmalloc(&st.counts, kCollideCounts + 2) || dmalloc(&st.scan_tmp, scan_ints(nc))) {
             *msg = "cell sort: device allocation failed";
             return PICGPU_OOM;
         }
         cudaMemsetAsync(st.scan_tmp, 0, scan_ints(nc) * sizeof(int), stream);
-        cudaMemsetAsync(st.overflow, 0, sizeof(int), stream);
     }
     CollideArgs a{};
     a.m = m;
@@ -2591,11 +2599,9 @@ int sort_species(CollideState& st, const DMesh& m, int s, const DSpecies& src, c
     // list position; deposits are integer sums and the push is per particle
     const int e = occupancy(st, a, s, msg, launches, st.enabled != 0);
     if (e) return e;
-    int total = 0, err = 0;
+    int total = 0;
     cudaMemcpyAsync(&total, st.cell_start + size_t(s) * (nc + 1) + nc, sizeof(int), cudaMemcpyDeviceToHost, stream);
-    cudaMemcpyAsync(&err, st.overflow, sizeof(int), cudaMemcpyDeviceToHost, stream);
-    if (cudaStreamSynchronize(stream) != cudaSuccess || err) {
-        if (err) cudaMemsetAsync(st.overflow, 0, sizeof(int), stream);
+    if (cudaStreamSynchronize(stream) != cudaSuccess) {
         *msg = "cell sort failed";
         return PICGPU_CUDA_ERROR;
     }
@@ -2846,19 +2852,17 @@ void launch_append(CollideState& st, const CollideArgs& a, long n, const int* us
     ScanState* scan = reinterpret_cast<ScanState*>(st.stage_scan);
     if (a.mixed)
         append_secondaries_kernel<float><<<scan_blocks(n), kScanThreads, 0, a.stream>>>(
-            st.flags, st.stage, n, used_dev, mask, T[0], T[1], added, scan, st.overflow);
+            st.flags, st.stage, n, used_dev, mask, T[0], T[1], added, scan, st.scan_polls, st.overflow);
     else
         append_secondaries_kernel<double><<<scan_blocks(n), kScanThreads, 0, a.stream>>>(
-            st.flags, st.stage, n, used_dev, mask, T[0], T[1], added, scan, st.overflow);
+            st.flags, st.stage, n, used_dev, mask, T[0], T[1], added, scan, st.scan_polls, st.overflow);
     *launches += 1;
 }
 
-// Reads back all counters, the numbers appended and the error flag; adds the
-// appended parcels to newn.
+// Reads back all counters and the numbers appended; adds the appended parcels to
+// newn.
 int read_counts(CollideState& st, const CollideArgs& a, u64 (&h)[kCollideCounts + 2], long newn[], std::string* msg) {
-    int err = 0;
     cudaMemcpyAsync(h, st.counts, sizeof h, cudaMemcpyDeviceToHost, a.stream);
-    cudaMemcpyAsync(&err, st.overflow, sizeof err, cudaMemcpyDeviceToHost, a.stream);
     if (cudaStreamSynchronize(a.stream) != cudaSuccess) {
         *msg = "collision step failed";
         return PICGPU_CUDA_ERROR;
@@ -2875,11 +2879,6 @@ int read_counts(CollideState& st, const CollideArgs& a, u64 (&h)[kCollideCounts 
             }
             newn[s] += long(h[kCollideCounts + bit]);
         }
-    if (err) {
-        cudaMemsetAsync(st.overflow, 0, sizeof(int), a.stream);
-        *msg = "collision step: a prefix sum's wait ran out";
-        return PICGPU_CUDA_ERROR;
-    }
     return PICGPU_OK;
 }
 
@@ -2919,7 +2918,7 @@ int mcc_parcels(CollideState& st, const CollideArgs& a, long newn[], std::string
     M.overflow = st.overflow;
     M.n_live = st.n_live;
     mcc_parcel_count_kernel<<<(nc + 255) / 256, 256, 0, a.stream>>>(M, st.ncand);
-    exclusive_scan(st.ncand, st.cand_off, nc, st.scan_tmp, st.overflow, a.stream, launches);
+    exclusive_scan(st.ncand, st.cand_off, nc, st.scan_tmp, st.scan_polls, a.stream, launches);
     int total = 0;
     cudaMemcpyAsync(&total, st.cand_off + nc, sizeof(int), cudaMemcpyDeviceToHost, a.stream);
     if (cudaStreamSynchronize(a.stream) != cudaSuccess) { *msg = "MCC: candidate count failed"; return PICGPU_CUDA_ERROR; }
@@ -3037,7 +3036,7 @@ int run_collisions(CollideState& st, const CollideArgs& a, int64_t counts[kColli
         mcc_count_kernel<<<(nc + 255) / 256, 256, 0, a.stream>>>(M, st.ncand);
         if (mcc_only)
             launch_order(nc, a.n[es], M.e_start, st.idx[es], st.sel[es], st.ncand, a.stream, launches);
-        exclusive_scan(st.ncand, st.cand_off, nc, st.scan_tmp, st.overflow, a.stream, launches);
+        exclusive_scan(st.ncand, st.cand_off, nc, st.scan_tmp, st.scan_polls, a.stream, launches);
         int total = 0;
         cudaMemcpyAsync(&total, st.cand_off + nc, sizeof(int), cudaMemcpyDeviceToHost, a.stream);
         if (cudaStreamSynchronize(a.stream) != cudaSuccess) { *msg = "MCC: candidate count failed"; return PICGPU_CUDA_ERROR; }
@@ -3153,7 +3152,7 @@ int run_collisions_device(CollideState& st, const CollideArgs& a, int* n_dev, in
         cudaMemsetAsync(st.cell_cursor, 0, (nc + 1) * sizeof(int), a.stream);
         const long cap = a.cap[s];
         count_cells_kernel<<<grid_of(cap, 256), 256, 0, a.stream>>>(a.sp[s].tet, int(cap), cnt, n_dev + s);
-        exclusive_scan(cnt, start, nc, st.scan_tmp, st.overflow, a.stream, launches);
+        exclusive_scan(cnt, start, nc, st.scan_tmp, st.scan_polls, a.stream, launches);
         scatter_cells_kernel<<<grid_of(cap, 256), 256, 0, a.stream>>>(a.sp[s].tet, int(cap), start, st.cell_cursor,
                                                                       st.idx[s], n_dev + s);
         *launches += 2;
@@ -3177,7 +3176,7 @@ int run_collisions_device(CollideState& st, const CollideArgs& a, int* n_dev, in
         mcc_count_kernel<<<(nc + 255) / 256, 256, 0, a.stream>>>(M, st.ncand);
         if (mcc_lists_only(cfg))
             launch_order(nc, a.n[es], M.e_start, st.idx[es], st.sel[es], st.ncand, a.stream, launches);
-        exclusive_scan(st.ncand, st.cand_off, nc, st.scan_tmp, st.overflow, a.stream, launches);
+        exclusive_scan(st.ncand, st.cand_off, nc, st.scan_tmp, st.scan_polls, a.stream, launches);
         if (a.mixed && !M.relativistic && M.xs32) launch_mcc_fp32(M, a.sp[es], st.stage, st.mcc_block, a.stream);
         else if (a.mixed) mcc_kernel<float><<<(nc + st.mcc_block - 1) / st.mcc_block, st.mcc_block, 0, a.stream>>>(M, a.sp[es], st.stage);
         else mcc_kernel<double><<<(nc + st.mcc_block - 1) / st.mcc_block, st.mcc_block, 0, a.stream>>>(M, a.sp[es], st.stage);
@@ -3478,7 +3477,7 @@ int merge_select(CollideState& st, const CollideArgs& a, int li, int s, long lon
     M.kin = st.mkin;
     if (a.mixed) merge_kernel<float><<<(nc + 127) / 128, 128, 0, a.stream>>>(M);
     else merge_kernel<double><<<(nc + 127) / 128, 128, 0, a.stream>>>(M);
-    exclusive_scan(st.mcount, st.moff, nc, st.scan_tmp, st.overflow, a.stream, launches);
+    exclusive_scan(st.mcount, st.moff, nc, st.scan_tmp, st.scan_polls, a.stream, launches);
     *launches += 1;
     int t = 0;
     if (cudaMemcpyAsync(&t, st.moff + nc, sizeof(int), cudaMemcpyDeviceToHost, a.stream) != cudaSuccess ||

@@ -102,6 +102,7 @@ struct CollideState {
     int* cell_count = nullptr;
     int* cell_cursor = nullptr;
     int* scan_tmp = nullptr;      // state of the prefix sums over the cells
+    unsigned scan_polls = 1u << 21;   // of a prefix sum's block, before it adds up by itself
     // kCollideCounts counters, then the electrons and ions appended:
     // candidates, elastic, excitation, ionisation, coulomb pairs,
     // ion candidates, ion elastic, ion charge exchange
@@ -116,7 +117,7 @@ struct CollideState {
     int* flags = nullptr;                  // per staging slot: 1 electron, 2 ion to append
     int* stage_scan = nullptr;             // state of their prefix sums
     long stage_cap = 0;
-    int* overflow = nullptr;                // staging or store overflow (device-driven step)
+    int* overflow = nullptr;                // staging or store overflow (read by the device-driven step)
     double svmax_init = 0.0;                // initial (sigma v)_max of the electron MCC
     double* psvmax = nullptr;               // electron - neutral parcel (sigma_T c_R)_max per cell
     double* premainder = nullptr;           // and its collision remainder per cell

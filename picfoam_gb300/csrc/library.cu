@@ -3028,6 +3028,13 @@ picgpu_status picgpu_test_pcg_ranks(picgpu_ctx* c, int ranks) {
     return PICGPU_OK;
 }
 
+picgpu_status picgpu_test_scan_polls(picgpu_ctx* c, unsigned polls) {
+    if (!c) return PICGPU_INVALID_ARG;
+    c->coll.scan_polls = polls;
+    drop_graphs(c);
+    return PICGPU_OK;
+}
+
 picgpu_status picgpu_timer_start(picgpu_ctx* c) {
     if (!c) return PICGPU_INVALID_ARG;
     if (!c->timer[0]) {
