@@ -704,15 +704,21 @@ void configure(const PcgPlan& p, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* a
     cfg->numAttrs = 1;
 }
 
+// Dynamic shared memory of a block with `slots` chunks of its own (kSmem).
+constexpr int smem_bytes(int slots) { return slots * (kSums * 256 + kVecs * kChunk) * int(sizeof(double)); }
+
 cudaError_t prepare(PcgPlan* plan, int sm_count, bool uniform) {
     const int slots = (plan->chunks + plan->clusters - 1) / plan->clusters, per = 256 / plan->split;
-    int doubles = plan->split > 1 ? 8 * 256 : kSums * slots * 256;
-    if (slots > 1) doubles += slots * kVecs * kChunk;
-    else if (plan->split > 1) doubles += 3 * kItems * per;
+    int doubles = plan->split > 1 ? 8 * 256 : kSums * 256;
+    if (plan->split > 1) doubles += 3 * kItems * per;
     else if (plan->alone) doubles += 3 * 256;
-    plan->smem = doubles * int(sizeof(double));
+    plan->smem = slots > 1 ? smem_bytes(slots) : doubles * int(sizeof(double));
     const Kernel k = kernel_of(*plan, uniform);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, plan->smem);
+    cudaError_t e = cudaSuccess;
+    // the limit belongs to the function, not to this plan: always the largest
+    // plan's, so that a smaller one does not take it from a context in use
+    if (slots > 1)
+        e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes(kSmemChunks));
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
