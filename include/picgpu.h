@@ -751,6 +751,9 @@ picgpu_status picgpu_solve_ldu_noalloc(int n_cells, const double* diag, const do
  * context is told to find.  Where that is not what it finds, it does nothing,
  * and the two-kernel iteration solves from then on. */
 picgpu_status picgpu_test_pcg_ranks(picgpu_ctx* ctx, int ranks);
+/* For tests: whether the waits of that solve give up after one look (meshes of
+ * more than 256 cells), so that it returns PICGPU_CUDA_ERROR. */
+picgpu_status picgpu_test_pcg_look_once(picgpu_ctx* ctx, int on);
 /* For tests: how often a block of the collision kernels' prefix sums looks for
  * its predecessors' sums before it adds up their items itself. */
 picgpu_status picgpu_test_scan_polls(picgpu_ctx* ctx, unsigned polls);

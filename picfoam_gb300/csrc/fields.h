@@ -35,6 +35,7 @@ struct PcgPlan {
     int chunks = 0;     // kChunk cells each
     int split = 1;      // blocks (one cluster) per chunk
     int ranks = 1;      // what the kernel is told of it
+    bool look_once = false;   // for tests: a wait gives up at once
     int clusters = 0;
     int smem = 0;
     bool alone = false; // one block, at most 256 cells

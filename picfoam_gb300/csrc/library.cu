@@ -3028,6 +3028,12 @@ picgpu_status picgpu_test_pcg_ranks(picgpu_ctx* c, int ranks) {
     return PICGPU_OK;
 }
 
+picgpu_status picgpu_test_pcg_look_once(picgpu_ctx* c, int on) {
+    if (!c) return PICGPU_INVALID_ARG;
+    c->pcg_plan.look_once = on != 0;
+    return PICGPU_OK;
+}
+
 picgpu_status picgpu_test_scan_polls(picgpu_ctx* c, unsigned polls) {
     if (!c) return PICGPU_INVALID_ARG;
     c->coll.scan_polls = polls;

@@ -64,7 +64,10 @@ namespace cg = cooperative_groups;
 namespace {
 
 constexpr int kScalarThreads = 96;          // warps G, R, D
-constexpr unsigned kSpinLimit = 1u << 22;   // polls of one wait, about a second
+// Polls of one wait before it gives up (8 times as many of an mbarrier): a poll
+// of a slot or counter is a load from L2, some 700 cycles, so this is seconds.
+// Tests run the kernels with waits that look once.
+constexpr unsigned kPolls = 1u << 22, kLookOnce = 2;
 // Where a block keeps r, p, s, w, u of its cells: registers (one chunk per
 // block) or shared memory (up to kSmemChunks).
 constexpr int kReg = 0, kSmem = 1;
@@ -128,7 +131,7 @@ __device__ __forceinline__ bool get(const double* p, unsigned, double* v) {
 }
 
 // Repeats ready() (uniform over the warp) until it holds; false when the limit
-// ran out or another block gave up.
+// (2 or more) ran out or another block gave up.
 template <class F>
 __device__ __forceinline__ bool wait_for(F ready, unsigned limit, const int* fail) {
     for (unsigned i = 1; i < limit; ++i) {
@@ -136,6 +139,17 @@ __device__ __forceinline__ bool wait_for(F ready, unsigned limit, const int* fai
         if ((i & 1023u) == 0 && *static_cast<const volatile int*>(fail)) break;
     }
     return false;
+}
+
+__device__ __forceinline__ bool phase_done(unsigned bar, unsigned parity) {
+    unsigned there;
+    asm volatile(
+        "{\n.reg .pred p;\nmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n}"
+        : "=r"(there)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return there != 0u;
 }
 
 __device__ __forceinline__ unsigned smem(const void* p) { return unsigned(__cvta_generic_to_shared(p)); }
@@ -151,7 +165,7 @@ constexpr int sums_per_lane(int S) { return S == 8 ? 1 : S == 4 ? 2 : S == 2 ? 3
 // One warp: the sum over nb chunk sums in the order of final_sum +
 // block_tree, without the additions of zeros (which change nothing); valid in
 // every lane.  *ok turns false when a sum did not come.
-template <int K, class Part>
+template <int K, unsigned Polls, class Part>
 __device__ __forceinline__ double warp_final_sum(const Part* part, int nb, unsigned pass, const int* fail, bool* ok) {
     const int lane = threadIdx.x & 31;
     double v[K];
@@ -170,7 +184,7 @@ __device__ __forceinline__ double warp_final_sum(const Part* part, int nb, unsig
                              }
                              return sizeof(Part) == sizeof(double) || __all_sync(0xffffffffu, all);
                          },
-                         kSpinLimit, fail);
+                         Polls, fail);
 #pragma unroll
         for (int k = 0; k < K; ++k)
             if (i0 == 0) v[k] = p[k];
@@ -219,6 +233,46 @@ __device__ __forceinline__ double row(const DMesh& m, double diag, double xc, co
     return s;
 }
 
+// The end of a cluster's block: it leaves when no other can still send to it.
+// After a wait that ran out, copies may be on their way that nobody waited for;
+// a thread per barrier of a block that receives then waits for them.  How many
+// there are follows from the pass in which each block stopped: it had sent its
+// sums of gamma and r.r in the passes before it, of delta up to it and of b.b
+// once.  A block is at most a pass ahead of another, so at most one phase per
+// barrier is open, and it is armed; the bytes that nobody sent are counted off.
+// (Not inlined: the kernel's registers then are what they were without it; as a
+// part of its body it cost 27,000 cells 3 % of an iteration.)
+template <int S>
+__device__ __noinline__ void leave(u64 (*bars)[2], unsigned* last_pass, unsigned* drain, unsigned pass, bool done,
+                                   bool receives) {
+    constexpr unsigned kPhase = 256u * 8u;
+    const cg::cluster_group cl = cg::this_cluster();
+    const unsigned tid = threadIdx.x;
+    if (tid == 0) *last_pass = pass;
+    if (!done && tid < S) *cl.map_shared_rank(drain, int(tid)) = 1u;
+    cl.sync();
+    if (!*drain) return;
+    if (tid < 8 && receives) {
+        const unsigned q = tid >> 1, odd = tid & 1u, bar = smem(&bars[q][odd]);
+        auto sent = [&](unsigned last) {
+            return q == 3u ? 1u - odd : ((q == 2u) == (odd != 0u) ? last + 1u : last) / 2u;
+        };
+        unsigned used = sent(pass);   // phases that this block waited for
+        if (used > 0u && !phase_done(bar, (used - 1u) & 1u)) --used;
+        unsigned bytes = 0u;
+        for (int r = 0; r < S; ++r) bytes += kPhase / S * sent(*cl.map_shared_rank(last_pass, r));
+        bytes -= kPhase * used;
+        if (bytes > 0u) {
+            if (bytes < kPhase)
+                asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cta.b64 [%0], %1;" ::"r"(bar),
+                             "r"(kPhase - bytes)
+                             : "memory");
+            for (unsigned i = 0; i < kPolls && !phase_done(bar, used & 1u); ++i) {}
+        }
+    }
+    cl.sync();
+}
+
 struct Scalars {
     double g, rr, beta, t, alpha;
 };
@@ -233,12 +287,13 @@ __device__ __forceinline__ void bar_arrive(int id, int n) {
 // S blocks (a cluster) per chunk; I cells per thread: kItems when a block has
 // whole chunks, 1 when it shares one or is alone with at most 256 cells.
 // Threads [0, M) own the block's cells; warps G, R and D the scalars.
-template <bool Uniform, int Mode, int I, int S>
+template <bool Uniform, int Mode, int I, int S, unsigned Polls>
 __device__ __forceinline__ void pcg_body(const PcgArgs& A) {
     extern __shared__ double dyn[];   // sums; then kSmem: the vectors, I = 1: r, u, w of the block
     __shared__ Scalars scalars[2];    // in turn: a warp may still read one pass's while the next one's are written
     __shared__ double sc_rz, sc_bb, sc_lim;
     __shared__ __align__(8) u64 bars[4][2];   // S > 1: bytes received, per quantity, odd and even passes
+    __shared__ unsigned last_pass, drain;     // S > 1: see leave()
     const cg::cluster_group cl = cg::this_cluster();
     // Every address of a peer below counts on S blocks per cluster.  A launch
     // that formed other ones (a tool between this library and the driver that
@@ -298,6 +353,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& A) {
                      : "memory");
     };
     if (S > 1) {
+        if (tid == 0) drain = 0u;
         if (tid < 8) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem(&bars[tid / 2][tid % 2])) : "memory");
             asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -351,18 +407,8 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& A) {
     auto received = [&](int q, unsigned pass) {
         if (S == 1) return;
         const unsigned bar = smem(&bars[q][pass & 1u]), phase = (q == 2 ? pass - 1 : pass) >> 1;
-        const bool ok = wait_for(
-            [&] {
-                unsigned there;
-                asm volatile(
-                    "{\n.reg .pred p;\nmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n"
-                    "selp.u32 %0, 1, 0, p;\n}"
-                    : "=r"(there)
-                    : "r"(bar), "r"(phase & 1u)
-                    : "memory");
-                return bool(__all_sync(0xffffffffu, there != 0u));
-            },
-            8 * kSpinLimit, &st->fail);
+        const bool ok = wait_for([&] { return bool(__all_sync(0xffffffffu, phase_done(bar, phase & 1u))); },
+                                 8 * Polls, &st->fail);
         if (!ok) failed();
         else if (lane == 0) expect(q, pass);
     };
@@ -376,7 +422,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& A) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->bar[b]) : "memory");
                 return bool(__all_sync(0xffffffffu, int(v - ph * unsigned(clusters)) >= 0));
             },
-            kSpinLimit, &st->fail);
+            Polls, &st->fail);
         if (!ok) failed();
     };
     auto put_part = [&](int q, int ch, double v) {
@@ -404,8 +450,9 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& A) {
         bool ok = true;
         const long set = long(2 * q + int(ph & 1u)) * nb;
         const double v =
-            counted_sums ? warp_final_sum<8>(reinterpret_cast<const double*>(A.part) + set, nb, 0u, &st->fail, &ok)
-                         : warp_final_sum<sums_per_lane(S)>(A.part + set, nb, pass0 + ph, &st->fail, &ok);
+            counted_sums
+                ? warp_final_sum<8, Polls>(reinterpret_cast<const double*>(A.part) + set, nb, 0u, &st->fail, &ok)
+                : warp_final_sum<sums_per_lane(S), Polls>(A.part + set, nb, pass0 + ph, &st->fail, &ok);
         if (!ok) failed();
         return v;
     };
@@ -494,7 +541,7 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& A) {
                             }
                             return bool(__all_sync(0xffffffffu, all));
                         },
-                        kSpinLimit, &st->fail);
+                        Polls, &st->fail);
                     if (!ok) failed();
                 }
 #pragma unroll
@@ -662,18 +709,18 @@ __device__ __forceinline__ void pcg_body(const PcgArgs& A) {
             st->exits = 0u;
         }
     }
-    if (S > 1) cl.sync();   // no block leaves while another may still send to it
+    if (S > 1) leave<S>(bars, &last_pass, &drain, ph, done != 0, single || rank == 0);
 }
 
-template <bool Uniform, int Mode, int I>
+template <bool Uniform, int Mode, int I, unsigned Polls = kPolls>
 __global__ void __launch_bounds__(threads_of(I, 1)) pcg_kernel(PcgArgs A) {
-    pcg_body<Uniform, Mode, I, 1>(A);
+    pcg_body<Uniform, Mode, I, 1, Polls>(A);
 }
 
 // The cluster's size belongs to the kernel, so no launch can be without it.
-template <bool Uniform, int S>
+template <bool Uniform, int S, unsigned Polls = kPolls>
 __global__ void __cluster_dims__(S, 1, 1) __launch_bounds__(threads_of(1, S)) pcg_cluster_kernel(PcgArgs A) {
-    pcg_body<Uniform, kReg, 1, S>(A);
+    pcg_body<Uniform, kReg, 1, S, Polls>(A);
 }
 
 using Kernel = void (*)(PcgArgs);
@@ -690,7 +737,22 @@ Kernel kernel_of(const PcgPlan& p) {
     return p.clusters >= p.chunks ? pcg_kernel<Uniform, kReg, kItems> : pcg_kernel<Uniform, kSmem, kItems>;
 }
 
-Kernel kernel_of(const PcgPlan& p, bool uniform) { return uniform ? kernel_of<true>(p) : kernel_of<false>(p); }
+// The forms whose blocks wait for one another, with waits that look once.
+Kernel look_once(const PcgPlan& p) {
+    switch (p.split) {
+        case 8: return pcg_cluster_kernel<false, 8, kLookOnce>;
+        case 4: return pcg_cluster_kernel<false, 4, kLookOnce>;
+        case 2: return pcg_cluster_kernel<false, 2, kLookOnce>;
+        default: break;
+    }
+    return p.clusters >= p.chunks ? pcg_kernel<false, kReg, kItems, kLookOnce>
+                                  : pcg_kernel<false, kSmem, kItems, kLookOnce>;
+}
+
+Kernel kernel_of(const PcgPlan& p, bool uniform) {
+    if (p.look_once && !p.alone) return look_once(p);
+    return uniform ? kernel_of<true>(p) : kernel_of<false>(p);
+}
 
 void configure(const PcgPlan& p, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
     *cfg = cudaLaunchConfig_t{};
@@ -780,7 +842,12 @@ cudaError_t launch_pcg_solve(const DMesh& m, const PcgPlan& plan, const double* 
     cudaLaunchAttribute attr[1];
     configure(plan, &cfg, attr);
     cfg.stream = s;
-    return cudaLaunchKernelEx(&cfg, kernel_of(plan, m.lap_uniform != 0), A);
+    const Kernel k = kernel_of(plan, m.lap_uniform != 0);
+    if (plan.look_once)   // a kernel that prepare() has not seen
+        if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 smem_bytes(kSmemChunks)))
+            return e;
+    return cudaLaunchKernelEx(&cfg, k, A);
 }
 
 }  // namespace pgd

@@ -100,6 +100,8 @@ def load():
                                              F64P, P]
     lib.picgpu_test_pcg_ranks.restype = i
     lib.picgpu_test_pcg_ranks.argtypes = [P, i]
+    lib.picgpu_test_pcg_look_once.restype = i
+    lib.picgpu_test_pcg_look_once.argtypes = [P, i]
     lib.picgpu_test_scan_polls.restype = i
     lib.picgpu_test_scan_polls.argtypes = [P, C.c_uint]
     U16P = C.POINTER(C.c_uint16)
