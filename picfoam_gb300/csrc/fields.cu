@@ -468,9 +468,10 @@ __device__ __forceinline__ bool boundary_phi(const DMesh& m, const double* grad_
 
 template <bool Box>
 __global__ void grad_E_kernel(DMesh m, const double* __restrict__ phi, const double* __restrict__ grad_bc,
-                              double* __restrict__ E, float* __restrict__ E32) {
+                              double* __restrict__ E, float* __restrict__ E32, const int* __restrict__ skip) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= m.n_cells) return;
+    const bool keep = skip && *skip;
     double g[3] = {0.0, 0.0, 0.0};
     const double phic = phi[c];
     bool finite = true;
@@ -504,6 +505,7 @@ __global__ void grad_E_kernel(DMesh m, const double* __restrict__ phi, const dou
             for (int a = 0; a < 3; ++a) g[a] = g[a] + pf * (n[a] * area);
         }
     }
+    if (keep) return;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         const double e = -(Box ? divide_by(g[a], m.box_vol, m.box_rvol) : g[a] / m.vol[c]);
@@ -514,9 +516,10 @@ __global__ void grad_E_kernel(DMesh m, const double* __restrict__ phi, const dou
 
 __global__ void boundary_E_kernel(DMesh m, const double* __restrict__ phi,
                                   const double* __restrict__ grad_bc, const double* __restrict__ E,
-                                  double* __restrict__ Eb) {
+                                  double* __restrict__ Eb, const int* __restrict__ skip) {
     const int b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= m.n_bfaces) return;
+    const bool keep = skip && *skip;
     const int c = m.bf_cell[b];
     const int pa = m.bf_patch[b];
     const double* Ec = E + 3 * size_t(c);
@@ -524,13 +527,16 @@ __global__ void boundary_E_kernel(DMesh m, const double* __restrict__ phi,
     const double sn = pg::face_sn_grad(pg::face_rule(c_patchF.kind[pa], c_patchF.phi_bc[pa]), c_patchF.phi[pa],
                                        grad_bc[pa], c_patchF.rlc_k[pa], m.bf_delta[b], phi[c]);
     const double En = Ec[0] * n[0] + Ec[1] * n[1] + Ec[2] * n[2];
+    if (keep) return;
     for (int a = 0; a < 3; ++a) Eb[3 * size_t(b) + a] = (Ec[a] - En * n[a]) - sn * n[a];
 }
 
 __global__ void point_E_kernel(DMesh m, const double* __restrict__ E, const double* __restrict__ Eb,
-                               double* __restrict__ Ept, float* __restrict__ Ept32) {
+                               double* __restrict__ Ept, float* __restrict__ Ept32,
+                               const int* __restrict__ skip) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= m.n_points) return;
+    const bool keep = skip && *skip;
     double e[3] = {0.0, 0.0, 0.0};
     for (int k = m.pi_start[p]; k < m.pi_start[p + 1]; ++k) {
         const int s = m.pi_src[k];
@@ -539,6 +545,7 @@ __global__ void point_E_kernel(DMesh m, const double* __restrict__ E, const doub
 #pragma unroll
         for (int a = 0; a < 3; ++a) e[a] = e[a] + w * src[a];
     }
+    if (keep) return;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         Ept[3 * size_t(p) + a] = e[a];
@@ -671,11 +678,12 @@ void launch_of_residual(const DMesh& m, const double* b, const double* x, double
 }
 
 void launch_efield(const DMesh& m, const double* phi, const double* grad_bc, double* E, double* Eb,
-                   double* Ept, float* E32, float* Ept32, cudaStream_t s) {
-    if (m.box) grad_E_kernel<true><<<blocks(m.n_cells, 256), 256, 0, s>>>(m, phi, grad_bc, E, E32);
-    else grad_E_kernel<false><<<blocks(m.n_cells, 256), 256, 0, s>>>(m, phi, grad_bc, E, E32);
-    if (m.n_bfaces > 0) boundary_E_kernel<<<blocks(m.n_bfaces, 256), 256, 0, s>>>(m, phi, grad_bc, E, Eb);
-    point_E_kernel<<<blocks(m.n_points, 256), 256, 0, s>>>(m, E, Eb, Ept, Ept32);
+                   double* Ept, float* E32, float* Ept32, const int* skip, cudaStream_t s) {
+    if (m.box) grad_E_kernel<true><<<blocks(m.n_cells, 256), 256, 0, s>>>(m, phi, grad_bc, E, E32, skip);
+    else grad_E_kernel<false><<<blocks(m.n_cells, 256), 256, 0, s>>>(m, phi, grad_bc, E, E32, skip);
+    if (m.n_bfaces > 0)
+        boundary_E_kernel<<<blocks(m.n_bfaces, 256), 256, 0, s>>>(m, phi, grad_bc, E, Eb, skip);
+    point_E_kernel<<<blocks(m.n_points, 256), 256, 0, s>>>(m, E, Eb, Ept, Ept32, skip);
 }
 
 void launch_to_float(const double* a, float* b, long n, cudaStream_t s) {

@@ -98,8 +98,9 @@ void launch_pcg_iteration(const DMesh& m, double* x, double* r, double* u, doubl
                           double* part, PcgState* st, int maxit, cudaStream_t s);
 void launch_of_residual(const DMesh& m, const double* b, const double* x, double* part, PcgState* st,
                         cudaStream_t s);
+// skip (optional): where it is not zero on the device, E stays as it is.
 void launch_efield(const DMesh& m, const double* phi, const double* grad_bc, double* E, double* Eb,
-                   double* Ept, float* E32, float* Ept32, cudaStream_t s);
+                   double* Ept, float* E32, float* Ept32, const int* skip, cudaStream_t s);
 void launch_to_float(const double* a, float* b, long n, cudaStream_t s);
 void launch_fill(double* a, long n, double v, cudaStream_t s);
 void launch_diagnostics(const int32_t* tet, const double* u0, const double* u1, const double* u2,

@@ -709,10 +709,11 @@ picgpu_status charge_update(picgpu_ctx* c) {
     return PICGPU_OK;
 }
 
-picgpu_status efield(picgpu_ctx* c) {
+// skip (optional): where it is not zero on the device, the field stays as it is.
+picgpu_status efield(picgpu_ctx* c, const int* skip = nullptr) {
     PhaseScope ps(c, PICGPU_PHASE_EFIELD);
     pgd::launch_efield(c->dm, c->phi, c->grad_bc, c->E, c->Eb, c->Ept, c->mixed ? c->E32 : nullptr,
-                       c->mixed ? c->Ept32 : nullptr, c->stream);
+                       c->mixed ? c->Ept32 : nullptr, skip, c->stream);
     c->launches += c->dm.n_bfaces > 0 ? 3 : 2;
     if (c->Ec4) {
         pgd::launch_corner_E(c->dm, c->E32, c->Ept32, c->Ec4, c->stream);
@@ -792,7 +793,7 @@ picgpu_status solve_jacobi(picgpu_ctx* c, double tol, int maxit, bool learned) {
     CK(cudaMemcpyAsync(c->st_host, c->st, sizeof(pgd::PcgState), cudaMemcpyDeviceToHost, c->stream));
     if (learned && c->ws) {
         CK(cudaStreamSynchronize(c->stream));
-        if (c->st_host->fail == pgd::kPcgShape) return PICGPU_OK;   // solved again, by the other path
+        if (c->st_host->fail) return PICGPU_OK;   // this potential is no sample
         CK(c->ws->after(c->dm, c->phi, c->st_host->iters, c->stream));
     }
     return PICGPU_OK;
@@ -833,7 +834,8 @@ picgpu_status poisson(picgpu_ctx* c, picgpu_step_stats* stats, bool learned = fa
             return s;
         }
     }
-    if ((s = efield(c))) return s;
+    // not from the potential of a solve that gave up, which the host sees behind it
+    if ((s = efield(c, !c->mg && c->pcg_plan.fits ? &c->st->fail : nullptr))) return s;
     CK(cudaStreamSynchronize(c->stream));
     if (!c->mg && c->pcg_plan.fits && c->st_host->fail) {
         const int why = c->st_host->fail;

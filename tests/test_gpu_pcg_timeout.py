@@ -35,3 +35,30 @@ def test_a_wait_that_runs_out(gpu, n):
         rho = rho[::-1].copy()
     g.close()
     o.close()
+
+
+@pytest.mark.parametrize("learned", [False, True])
+def test_a_failed_solve_leaves_field_and_network(gpu, learned):
+    case = cases.electrode_box(n_cells=32, per_cell=4, seed=5)
+    case.cfg.learned.enabled = 1 if learned else 0
+    case.cfg.learned.train_steps = 20
+    case.cfg.learned.train_iters = 2
+    look_once = native.load().picgpu_test_pcg_look_once
+    g = cases.build(case, backend=gpu)
+    for _ in range(4):
+        before = g.step(1)
+    # a field that is not the gradient of the potential at hand
+    kinds = (abi.FIELD_E_CELL, abi.FIELD_E_POINT)
+    E = [1.5 * g.field(k) for k in kinds]
+    for k, v in zip(kinds, E):
+        g.set_field(k, v)
+    assert look_once(g._h, 1) == abi.OK
+    with pytest.raises(PicError) as e:
+        g.step(1)
+    assert e.value.status == abi.CUDA_ERROR
+    assert all(np.array_equal(v, g.field(k)) for k, v in zip(kinds, E))
+    assert look_once(g._h, 0) == abi.OK
+    after = g.step(1)
+    assert not np.array_equal(E[0], g.field(abi.FIELD_E_CELL))
+    assert after.learned_samples == before.learned_samples + (1 if learned else 0)
+    g.close()
