@@ -306,11 +306,12 @@ __global__ void __launch_bounds__(256) mg_rz_kernel(Lv L, const float* __restric
 // aggregate had an eighth of the threads in flight and eight stencils in a
 // row each; 2.7 us at 64^3 voxels now, 9.2 at 128^3.)
 template <bool Uniform>
-__global__ void __launch_bounds__(256) mg_restrict_kernel(Lv F, Lv Cl, int sx, int sy, int sz,
+__global__ void __launch_bounds__(256) mg_restrict_kernel(Lv F, Lv Cl, int sx, int sy, int sz, int y_first,
                                                           const float* __restrict__ b, const float* __restrict__ x,
                                                           float* __restrict__ bc) {
     after_previous();
-    const int i = blockIdx.x * 16 + (threadIdx.x & 15), j = blockIdx.y * 16 + (threadIdx.x >> 4);
+    const int i = (y_first ? blockIdx.y : blockIdx.x) * 16 + (threadIdx.x & 15);
+    const int j = (y_first ? blockIdx.x : blockIdx.y) * 16 + (threadIdx.x >> 4);
     const int ck = blockIdx.z;
     const bool in = i < F.X && j < F.Y;
     auto xv = [&](int w) { return x[w]; };
@@ -1008,12 +1009,16 @@ int MultigridPCG::vcycle(int l, cudaStream_t s) {
     }
     const MgLevel& C = lv_[l + 1];
     const Lv cv = view(C);
-    const dim3 rg((L.n[0] + 15) / 16, (L.n[1] + 15) / 16, C.n[2]);
+    // the longer of x and y along the grid's x, which alone takes more than 65535
+    // tiles (a plane has fewer than 2^31 voxels)
+    const int y_first = L.n[1] > L.n[0];
+    const unsigned tx = (L.n[0] + 15) / 16, ty = (L.n[1] + 15) / 16;
+    const dim3 rg(y_first ? ty : tx, y_first ? tx : ty, C.n[2]);
     const int sx = L.fac[0] - 1, sy = L.fac[1] - 1, sz = L.fac[2] - 1;
     if (L.uniform)
-        launch(mg_restrict_kernel<true>, rg, 256, s, v, cv, sx, sy, sz, L.b, cur, C.b);
+        launch(mg_restrict_kernel<true>, rg, 256, s, v, cv, sx, sy, sz, y_first, L.b, cur, C.b);
     else
-        launch(mg_restrict_kernel<false>, rg, 256, s, v, cv, sx, sy, sz, L.b, cur, C.b);
+        launch(mg_restrict_kernel<false>, rg, 256, s, v, cv, sx, sy, sz, y_first, L.b, cur, C.b);
     ++launched;
     launched += vcycle(l + 1, s);
     Interp P{};
