@@ -69,10 +69,12 @@ struct Lv {
 };
 
 // What the prolongation from a level's aggregates needs: their grid, the
-// aggregation shifts, periodic axes and edge factors.
+// aggregation shifts, periodic axes, edge factors and neighbour weights.
 struct Interp {
     int n[3], s[3], cyc[3];
     float edge[6];
+    int fine[3];
+    float w_first[3], w_last[3][3];
 };
 
 constexpr int kZB = 8;
@@ -332,16 +334,33 @@ __global__ void __launch_bounds__(256) mg_restrict_kernel(Lv F, Lv Cl, int sx, i
     if (in && !(sx && (i & 1)) && !(sy && (j & 1))) bc[(i >> sx) + Cl.X * ((j >> sy) + Cl.Y * ck)] = s;
 }
 
+// Weight of the neighbour aggregate for fine voxel i along axis a.  (Selects: with
+// branches or indexed constants an iteration at 33^3 took 14 us longer, and
+// where all weights are 1/4 they are left out.)
+template <bool Regular>
+__device__ __forceinline__ float neighbour_weight(const Interp& P, int a, int i) {
+    if (Regular) return 0.25f;
+    const int k = P.fine[a] - i;
+    float w = i == 0 ? P.w_first[a] : 0.25f;
+    w = k == 3 ? P.w_last[a][0] : w;
+    w = k == 2 ? P.w_last[a][1] : w;
+    return k == 1 ? P.w_last[a][2] : w;
+}
+
 // The coarse correction at fine voxel (i, j, k), interpolated linearly between
-// the aggregate centres (weights 3/4 and 1/4 per paired axis).  Beyond a
+// the aggregate centres (weights 3/4 and 1/4 per paired axis, others where an
+// odd count leaves the last aggregate narrower than the rest).  Beyond a
 // non-periodic edge the coarse value is edge x its mirror image: -1 where the
 // potential is given there (the correction is zero on that face), +1 where
 // its gradient is.
+template <bool Regular>
 __device__ __forceinline__ float coarse_at(const Interp& P, int i, int j, int k, const float* __restrict__ xc) {
     const int ci = i >> P.s[0], cj = j >> P.s[1], ck = k >> P.s[2];
     // the neighbour aggregate on the child's side, per axis
     int ni = ci + ((i & 1) ? 1 : -1), nj = cj + ((j & 1) ? 1 : -1), nk = ck + ((k & 1) ? 1 : -1);
-    float wi = 0.25f, wj = 0.25f, wk = 0.25f, ai = 0.75f, aj = 0.75f, ak = 0.75f;
+    float wi = neighbour_weight<Regular>(P, 0, i), wj = neighbour_weight<Regular>(P, 1, j),
+          wk = neighbour_weight<Regular>(P, 2, k);
+    float ai = 1.f - wi, aj = 1.f - wj, ak = 1.f - wk;
     if (!P.s[0]) { ni = ci; wi = 0.f; ai = 1.f; }
     else if (ni < 0) { if (P.cyc[0]) ni = P.n[0] - 1; else { ni = ci; wi *= P.edge[0]; } }
     else if (ni >= P.n[0]) { if (P.cyc[0]) ni = 0; else { ni = ci; wi *= P.edge[1]; } }
@@ -362,19 +381,20 @@ __device__ __forceinline__ float coarse_at(const Interp& P, int i, int j, int k,
 }
 
 // x += scale * (coarse correction) on the active voxels.
+template <bool Regular>
 __global__ void __launch_bounds__(256) mg_prolong_kernel(Lv F, Interp P, const float* __restrict__ xc,
                                                          float* __restrict__ x, float scale) {
     after_previous();
     int i, j, k, v;
     if (!coords(F, i, j, k, v)) return;
     if (F.inv[v] == 0.f) return;
-    x[v] = fmaf(scale, coarse_at(P, i, j, k, xc), x[v]);
+    x[v] = fmaf(scale, coarse_at<Regular>(P, i, j, k, xc), x[v]);
 }
 
 // The prolongation inside the first post sweep: x' = x + scale * (coarse
 // correction) on the active voxels (zero on holes) is formed at the seven
 // stencil points, y = x' + omega D^-1 (b - A x').
-template <bool Uniform>
+template <bool Uniform, bool Regular>
 __global__ void __launch_bounds__(256) mg_prolong_smooth_kernel(Lv L, Interp P, const float* __restrict__ xc,
                                                                 const float* __restrict__ b,
                                                                 const float* __restrict__ x, float* __restrict__ y,
@@ -384,7 +404,7 @@ __global__ void __launch_bounds__(256) mg_prolong_smooth_kernel(Lv L, Interp P, 
     if (!coords(L, i, j, k, v)) return;
     auto at = [&](int w, int wi, int wj, int wk) {
         if (L.inv[w] == 0.f) return 0.f;
-        return fmaf(scale, coarse_at(P, wi, wj, wk, xc), x[w]);
+        return fmaf(scale, coarse_at<Regular>(P, wi, wj, wk, xc), x[w]);
     };
     // neighbours with the periodic wrap; across a non-periodic edge the point
     // is v itself with a zero coefficient
@@ -687,6 +707,20 @@ long vnbr(const HostLevel& L, int i, int j, int k, int f) {
     return vidx(L, q[0], q[1], q[2]);
 }
 
+// The neighbour aggregate's weight for fine voxel i of an axis with n voxels
+// between the positions x[0..n]: linear between the aggregates' centres, mirrored
+// at a non-periodic end.
+double linear_weight(const std::vector<double>& x, int n, bool cyc, int i) {
+    const int m = (n + 1) / 2, I = i / 2;
+    auto centre = [&](int J) { return 0.5 * (x[2 * J] + x[std::min(2 * J + 2, n)]); };
+    const double d = 0.5 * (x[i] + x[i + 1]) - centre(I), length = x[n] - x[0];
+    if (d == 0.0) return 0.0;
+    double to;   // the distance to the neighbour's centre
+    if (d < 0.0) to = I > 0 ? centre(I) - centre(I - 1) : cyc ? centre(0) + length - centre(m - 1) : 2.0 * (centre(0) - x[0]);
+    else to = I < m - 1 ? centre(I + 1) - centre(I) : cyc ? centre(0) + length - centre(m - 1) : 2.0 * (x[n] - centre(m - 1));
+    return std::fabs(d) / to;
+}
+
 // Gauss-Jordan inverse with partial pivoting (row-major, in place).
 bool invert(std::vector<double>& a, int n) {
     std::vector<double> inv(size_t(n) * n, 0.0);
@@ -799,6 +833,7 @@ bool MultigridPCG::init(const pg::HexMesh& m, const std::vector<double>& Mdiag, 
         Cl.diag.assign(Cl.V, 0.0);
         Cl.off.assign(6 * size_t(Cl.V), 0.0);
         Cl.act.assign(Cl.V, 0);
+        std::vector<int> members(Cl.V, 0);
         for (int k = 0; k < F.n[2]; ++k)
             for (int j = 0; j < F.n[1]; ++j)
                 for (int i = 0; i < F.n[0]; ++i) {
@@ -807,6 +842,7 @@ bool MultigridPCG::init(const pg::HexMesh& m, const std::vector<double>& Mdiag, 
                     const int ci = i / fa[0], cj = j / fa[1], ck = k / fa[2];
                     const long I = vidx(Cl, ci, cj, ck);
                     Cl.act[I] = 1;
+                    ++members[I];
                     Cl.diag[I] += F.diag[v];
                     for (int f = 0; f < 6; ++f) {
                         const double o = F.off[f * size_t(F.V) + v];
@@ -829,8 +865,23 @@ bool MultigridPCG::init(const pg::HexMesh& m, const std::vector<double>& Mdiag, 
                         }
                     }
                 }
-        for (long I = 0; I < Cl.V; ++I)
-            if (!Cl.act[I]) Cl.diag[I] = 1.0;
+        // The coupling of an aggregate to given potentials is twice as stiff as
+        // its distance to them says, and the correction scale makes up for it.  An
+        // aggregate that is not full is as close to them as its voxels are, so
+        // there it counts twice.  Iterations to 1e-10 without and with this and the
+        // weights of odd counts: 33^3 between walls 20 and 12, 33^3 with periodic,
+        // insulated and given sides 25 and 17 (21 with constant prolongation), 48^3
+        // periodic with a plate across 23 and 20 (18), 61 x 97 cells 17 and 11.
+        for (long I = 0; I < Cl.V; ++I) {
+            if (!Cl.act[I]) {
+                Cl.diag[I] = 1.0;
+                continue;
+            }
+            if (members[I] == fa[0] * fa[1] * fa[2]) continue;
+            double given = Cl.diag[I];
+            for (int f = 0; f < 6; ++f) given += Cl.off[f * size_t(Cl.V) + I];
+            if (given > 1e-9 * Cl.diag[I]) Cl.diag[I] += given;
+        }
         fac.push_back(fa);
         hl.push_back(std::move(Cl));
     }
@@ -870,15 +921,42 @@ bool MultigridPCG::init(const pg::HexMesh& m, const std::vector<double>& Mdiag, 
         return false;
     }
 
+    // the correction vanishes on a side whose potential is given (an RLC
+    // cathode's too, nearly) and is flat across one whose gradient is
+    for (int f = 0; f < 6; ++f) {
+        const auto& p = m.patches[f].p;
+        const int rule = pg::face_rule(p.kind, p.phi_bc);
+        const bool given = p.kind != PICGPU_PATCH_EMPTY && (rule == pg::kRuleFixed || rule == pg::kRuleRlc);
+        edge_[f] = given ? -1.f : 1.f;
+    }
     // upload
     lv_.resize(hl.size());
+    std::vector<double> pos_of[3];   // the level's voxel ends along each axis
+    for (int a = 0; a < 3; ++a)
+        for (int i = 0; i <= hl[0].n[a]; ++i) pos_of[a].push_back(i);
     for (size_t l = 0; l < hl.size(); ++l) {
         const HostLevel& H = hl[l];
         MgLevel& L = lv_[l];
+        L.regular = 1;
         for (int a = 0; a < 3; ++a) {
             L.n[a] = H.n[a];
             L.cyc[a] = H.cyc[a];
             L.fac[a] = l + 1 < hl.size() ? fac[l][a] : 1;
+            L.w_first[a] = 0.25f;
+            for (float& w : L.w_last[a]) w = 0.25f;
+            if (L.fac[a] == 1) continue;
+            // (33^3 insulated: 11 iterations with 1/4 at the far side, 13 with these)
+            if (H.cyc[a] || edge_[2 * a + 1] < 0.f) {
+                L.w_first[a] = float(linear_weight(pos_of[a], H.n[a], H.cyc[a], 0));
+                for (int i = std::max(0, H.n[a] - 3); i < H.n[a]; ++i)
+                    L.w_last[a][i - (H.n[a] - 3)] = float(linear_weight(pos_of[a], H.n[a], H.cyc[a], i));
+            }
+            L.regular = L.regular && L.w_first[a] == 0.25f && L.w_last[a][0] == 0.25f && L.w_last[a][1] == 0.25f &&
+                        L.w_last[a][2] == 0.25f;
+            std::vector<double> coarse;
+            for (int i = 0; i < H.n[a]; i += 2) coarse.push_back(pos_of[a][i]);
+            coarse.push_back(pos_of[a][H.n[a]]);
+            pos_of[a].swap(coarse);
         }
         L.V = H.V;
         std::vector<float> diag(H.V), inv(H.V), off(6 * size_t(H.V));
@@ -932,14 +1010,6 @@ bool MultigridPCG::init(const pg::HexMesh& m, const std::vector<double>& Mdiag, 
         vox[c] = int(vidx(hl[0], m.cell_ijk[3 * size_t(c)], m.cell_ijk[3 * size_t(c) + 1],
                           m.cell_ijk[3 * size_t(c) + 2]));
     const long V0 = hl[0].V;
-    // the correction vanishes on a side whose potential is given (an RLC
-    // cathode's too, nearly) and is flat across one whose gradient is
-    for (int f = 0; f < 6; ++f) {
-        const auto& p = m.patches[f].p;
-        const int rule = pg::face_rule(p.kind, p.phi_bc);
-        const bool given = p.kind != PICGPU_PATCH_EMPTY && (rule == pg::kRuleFixed || rule == pg::kRuleRlc);
-        edge_[f] = given ? -1.f : 1.f;
-    }
     // block partials: the widest reduction launch (cells, or the level-0 grid)
     const long nbmax = std::max<long>(pcg_blocks(m.n_cells), shape(lv_[0]).blocks);
     part_cap_ = 2 * nbmax + 8;
@@ -1026,6 +1096,9 @@ int MultigridPCG::vcycle(int l, cudaStream_t s) {
         P.n[a] = C.n[a];
         P.s[a] = L.fac[a] - 1;
         P.cyc[a] = C.cyc[a];
+        P.fine[a] = L.n[a];
+        P.w_first[a] = L.w_first[a];
+        for (int q = 0; q < 3; ++q) P.w_last[a][q] = L.w_last[a][q];
     }
     for (int f = 0; f < 6; ++f) P.edge[f] = edge_[f];
     // on small levels a launch costs more than forming the correction seven
@@ -1034,13 +1107,12 @@ int MultigridPCG::vcycle(int l, cudaStream_t s) {
     const bool fuse = L.V <= kFuseVoxels && set_.post >= 1 && !(l == 0 && set_.post == 1);
     const float scale = kLinear * float(set_.scale);
     if (fuse) {
-        if (L.uniform)
-            launch(mg_prolong_smooth_kernel<true>, sh.grid, sh.block, s, v, P, result(l + 1), L.b, cur, oth, scale, om);
-        else
-            launch(mg_prolong_smooth_kernel<false>, sh.grid, sh.block, s, v, P, result(l + 1), L.b, cur, oth, scale, om);
+        auto k = L.uniform ? (L.regular ? mg_prolong_smooth_kernel<true, true> : mg_prolong_smooth_kernel<true, false>)
+                           : (L.regular ? mg_prolong_smooth_kernel<false, true> : mg_prolong_smooth_kernel<false, false>);
+        launch(k, sh.grid, sh.block, s, v, P, result(l + 1), L.b, cur, oth, scale, om);
         std::swap(cur, oth);
     } else {
-        launch(mg_prolong_kernel, sh.grid, sh.block, s, v, P, result(l + 1), cur, scale);
+        launch(L.regular ? mg_prolong_kernel<true> : mg_prolong_kernel<false>, sh.grid, sh.block, s, v, P, result(l + 1), cur, scale);
     }
     ++launched;
     for (int it = fuse ? 1 : 0; it < set_.post; ++it) {

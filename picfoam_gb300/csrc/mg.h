@@ -51,6 +51,10 @@ struct MgLevel {
     int n[3];             // voxel grid
     int cyc[3];           // periodic axes
     int fac[3];           // aggregation factor towards the next level (1 or 2)
+    // weights of the neighbour aggregate in the prolongation from the next
+    // level: 1/4, but for the first voxel and the last three of an axis
+    int regular;          // 1/4 for those too
+    float w_first[3], w_last[3][3];
     long V;
     int uniform;          // every coupling between active voxels in direction f equals coef[f]
     float coef[6];
