@@ -754,6 +754,9 @@ picgpu_status picgpu_test_pcg_ranks(picgpu_ctx* ctx, int ranks);
 /* For tests: whether the waits of that solve give up after one look (meshes of
  * more than 256 cells), so that it returns PICGPU_CUDA_ERROR. */
 picgpu_status picgpu_test_pcg_look_once(picgpu_ctx* ctx, int on);
+/* For tests: the blocks of the FP32 mover for this many parcels, whose last step
+ * crossed this many faces, on a GPU of `sms` SMs. */
+int picgpu_test_move_blocks(int64_t parcels, double faces, int sms);
 /* For tests: how often a block of the collision kernels' prefix sums looks for
  * its predecessors' sums before it adds up their items itself. */
 picgpu_status picgpu_test_scan_polls(picgpu_ctx* ctx, unsigned polls);

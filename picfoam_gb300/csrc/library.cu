@@ -676,7 +676,9 @@ picgpu_status move_species(picgpu_ctx* c, bool deposit_only) {
         {
             PhaseScope ps(c, PICGPU_PHASE_MOVE);
             if (c->mixed) {
-                c->launches += pgd::launch_move_fp32(P, pgd::kMoveBlocks32 * c->sm_count, c->stream);
+                // the counters of this species' last step, which the host has read
+                const int blocks = pgd::move_blocks32(c->sp[s].n, double(c->counters_host[s].faces), c->sm_count);
+                c->launches += pgd::launch_move_fp32(P, blocks, c->stream);
             } else {
                 pgd::launch_move_fp64(P, c->sm_count, c->stream);
                 c->launches++;
@@ -1302,7 +1304,8 @@ picgpu_status pgd_collisions(picgpu_ctx* c, picgpu_step_stats* stats) {
             pgd::MoveParams P = move_params(c, s, true);
             P.first = int(old);
             if (c->mixed) {
-                c->launches += pgd::launch_move_fp32(P, pgd::kMoveBlocks32 * c->sm_count, c->stream);
+                c->launches +=
+                    pgd::launch_move_fp32(P, pgd::move_blocks32(newn[s] - old, 0.0, c->sm_count), c->stream);
             } else {
                 pgd::launch_move_fp64(P, c->sm_count, c->stream);
                 c->launches++;
@@ -3034,6 +3037,10 @@ picgpu_status picgpu_test_pcg_look_once(picgpu_ctx* c, int on) {
     if (!c) return PICGPU_INVALID_ARG;
     c->pcg_plan.look_once = on != 0;
     return PICGPU_OK;
+}
+
+int picgpu_test_move_blocks(int64_t parcels, double faces, int sms) {
+    return pgd::move_blocks32(long(parcels), faces, sms);
 }
 
 picgpu_status picgpu_test_scan_polls(picgpu_ctx* c, unsigned polls) {

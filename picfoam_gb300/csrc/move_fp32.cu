@@ -936,6 +936,12 @@ int launch_pusher(const MoveParams& P, int blocks, int chunk, bool cell, cudaStr
 
 }  // namespace
 
+int move_blocks32(long parcels, double faces, int sms) {
+    const bool many = parcels >= 72000L * sms;
+    const bool crossing = faces >= 10.0 * double(parcels) && faces >= 80000.0 * sms;
+    return (many || crossing ? 15 : 5) * sms;
+}
+
 // grid: the number of blocks to use (5 per SM are resident); each block takes one
 // contiguous chunk (a multiple of 256 particles) of [P.first, P.n).  With
 // P.n_dev set the counts are read on the device and all grid blocks launch.

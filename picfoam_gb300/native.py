@@ -102,6 +102,8 @@ def load():
     lib.picgpu_test_pcg_ranks.argtypes = [P, i]
     lib.picgpu_test_pcg_look_once.restype = i
     lib.picgpu_test_pcg_look_once.argtypes = [P, i]
+    lib.picgpu_test_move_blocks.restype = i
+    lib.picgpu_test_move_blocks.argtypes = [C.c_int64, C.c_double, i]
     lib.picgpu_test_scan_polls.restype = i
     lib.picgpu_test_scan_polls.argtypes = [P, C.c_uint]
     U16P = C.POINTER(C.c_uint16)
