@@ -28,6 +28,14 @@ extern "C" {
 picgpu_status picgpu_test_conv3d(int X, int Y, int Z, int cin1, int cin2, int up1, int cout, int relu,
                                  const uint16_t* in1, const uint16_t* in2, const uint16_t* w, float* out);
 
+/* The weight gradient of such a convolution: dw[27][cout][cin1+cin2] in FP32 =
+ * sum over the voxels of output gradient times shifted input.  The input is as
+ * above or, for 2 -> 16 channels, FP32 x32[X*Y*Z][2]; the output gradient is
+ * BF16 h[X*Y*Z][cout] or, for 16 -> 1, FP32 h32[X*Y*Z].  Any grid. */
+picgpu_status picgpu_test_conv3d_dw(int X, int Y, int Z, int cin1, int cin2, int up1, int cout, const uint16_t* in1,
+                                    const uint16_t* in2, const uint16_t* h, const float* x32, const float* h32,
+                                    float* dw);
+
 /* The warm-start network on its own (host buffers).  Grid X x Y x Z (x
  * fastest) must be a multiple of 4 per direction with X*Y*Z/64 a multiple of
  * 128.  Weights are FP32, all layers back to back in the order c1a c1b c2a

@@ -3,6 +3,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "picgpu_learned.h"
@@ -71,6 +72,44 @@ extern "C" picgpu_status picgpu_test_conv3d(int X, int Y, int Z, int cin1, int c
     } else if (cudaMemcpy(out, dout, size_t(V) * cout * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess) {
         return PICGPU_CUDA_ERROR;
     }
+    return PICGPU_OK;
+}
+
+extern "C" picgpu_status picgpu_test_conv3d_dw(int X, int Y, int Z, int cin1, int cin2, int up1, int cout,
+                                               const uint16_t* in1, const uint16_t* in2, const uint16_t* h,
+                                               const float* x32, const float* h32, float* dw) {
+    if (X <= 0 || Y <= 0 || Z <= 0 || cin1 < 0 || cin2 < 0 || cout <= 0 || !dw || (x32 ? cin1 + cin2 != 2 : !in1) ||
+        (!x32 && cin2 > 0 && !in2) || (!h32 && !h))
+        return PICGPU_INVALID_ARG;
+    if (!x32 && (cin1 % 8 != 0 || cin2 % 8 != 0 || (up1 && (X % 2 || Y % 2 || Z % 2)))) return PICGPU_INVALID_ARG;
+    const size_t V = size_t(X) * Y * Z, V1 = up1 ? V / 8 : V, nw = size_t(27) * cout * (cin1 + cin2);
+    DeviceBuffers B;
+    bool copied = true;
+    auto upload = [&](auto* src, size_t n) -> decltype(src) {
+        using T = std::remove_const_t<std::remove_pointer_t<decltype(src)>>;
+        if (!src || n == 0) return nullptr;
+        T* p = B.alloc<T>(n);
+        copied = copied && p && cudaMemcpy(p, src, n * sizeof(T), cudaMemcpyHostToDevice) == cudaSuccess;
+        return p;
+    };
+    const auto* d1 = reinterpret_cast<const __nv_bfloat16*>(upload(x32 ? nullptr : in1, V1 * cin1));
+    const auto* d2 = reinterpret_cast<const __nv_bfloat16*>(upload(x32 ? nullptr : in2, V * cin2));
+    const auto* dh = reinterpret_cast<const __nv_bfloat16*>(upload(h32 ? nullptr : h, V * cout));
+    const float* dx = upload(x32, 2 * V);
+    const float* dg = upload(h32, V);
+    float* out = B.alloc<float>(nw);
+    int* derr = B.alloc<int>(1);
+    if (!copied || !out || !derr || cudaMemset(out, 0, nw * sizeof(float)) != cudaSuccess ||
+        cudaMemset(derr, 0, sizeof(int)) != cudaSuccess)
+        return PICGPU_CUDA_ERROR;
+    const pgd::ConvSrc s1{d1, x32 ? 0 : cin1, up1}, s2{d2, x32 ? 0 : cin2, 0};
+    const cudaError_t e = pgd::launch_dw_tc(cin1 + cin2, cout, {X, Y, Z}, dh, dg, s1, s2, dx, out, derr, 0);
+    if (e == cudaErrorInvalidValue) return PICGPU_NOT_SUPPORTED;
+    int herr = 0;
+    if (e != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
+        cudaMemcpy(&herr, derr, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess || herr ||
+        cudaMemcpy(dw, out, nw * sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)
+        return PICGPU_CUDA_ERROR;
     return PICGPU_OK;
 }
 

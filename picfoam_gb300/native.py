@@ -110,6 +110,8 @@ def load():
     F32P = C.POINTER(C.c_float)
     lib.picgpu_test_conv3d.restype = i
     lib.picgpu_test_conv3d.argtypes = [i, i, i, i, i, i, i, i, U16P, U16P, U16P, F32P]
+    lib.picgpu_test_conv3d_dw.restype = i
+    lib.picgpu_test_conv3d_dw.argtypes = [i, i, i, i, i, i, i, U16P, U16P, U16P, F32P, F32P, F32P]
     lib.picgpu_ensemble_create.restype = i
     lib.picgpu_ensemble_create.argtypes = [C.POINTER(abi.MeshDesc), i, C.POINTER(abi.Config), PP]
     lib.picgpu_ensemble_set_efield.restype = i
