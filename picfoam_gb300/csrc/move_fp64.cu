@@ -205,9 +205,9 @@ __device__ __forceinline__ double leg(const MoveParams& P, const TetConst& T, co
         for (int a = 0; a < 3; ++a) {
             if (!P.m.empty[a]) continue;
             Ut[a] = 0.0;
-            const double x = PC<double>::cc(P, s.cell, a) + s.y[1] * off[3 * T.tri[s.tet][0] + a] +
+            const double x = P.m.cc[3 * size_t(s.cell) + a] + s.y[1] * off[3 * T.tri[s.tet][0] + a] +
                              s.y[2] * off[3 * T.tri[s.tet][1] + a] + s.y[3] * off[3 * T.tri[s.tet][2] + a];
-            dev[a] = x - PC<double>::centre(P, a);
+            dev[a] = x - P.m.mesh_centre[a];
         }
     }
     const double f = 1.0 - sf;

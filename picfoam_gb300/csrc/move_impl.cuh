@@ -28,19 +28,11 @@ template <> struct PC<double> {
         }
         return P.q * zf * half_dt / P.mass;
     }
-    static __device__ __forceinline__ double centre(const MoveParams& P, int a) { return P.m.mesh_centre[a]; }
-    static __device__ __forceinline__ double cc(const MoveParams& P, int c, int a) {
-        return P.m.cc[3 * size_t(c) + a];
-    }
 };
 template <> struct PC<float> {
     static __device__ __forceinline__ float B(const MoveParams& P, int a) { return P.B_f[a]; }
     static __device__ __forceinline__ float qdm(const MoveParams& P, float half_dt, float zf) {
         return P.qm_f * zf * half_dt;
-    }
-    static __device__ __forceinline__ float centre(const MoveParams& P, int a) { return P.centre_f[a]; }
-    static __device__ __forceinline__ float cc(const MoveParams& P, int c, int a) {
-        return P.m.cc32[3 * size_t(c) + a];
     }
 };
 
@@ -97,15 +89,6 @@ template <> __device__ __forceinline__ const float* e_cell<float>(const MovePara
 template <class Real> __device__ __forceinline__ const Real* e_point(const MoveParams& P);
 template <> __device__ __forceinline__ const double* e_point<double>(const MoveParams& P) { return P.Ept; }
 template <> __device__ __forceinline__ const float* e_point<float>(const MoveParams& P) { return P.Ept32; }
-template <class Real> __device__ __forceinline__ const Real* tetinv(const DMesh& m);
-template <> __device__ __forceinline__ const double* tetinv<double>(const DMesh& m) { return m.tetinv; }
-template <> __device__ __forceinline__ const float* tetinv<float>(const DMesh& m) { return m.tetinv32; }
-template <class Real> __device__ __forceinline__ const Real* offsets(const DMesh& m);
-template <> __device__ __forceinline__ const double* offsets<double>(const DMesh& m) { return m.offset; }
-template <> __device__ __forceinline__ const float* offsets<float>(const DMesh& m) { return m.offset32; }
-template <class Real> __device__ __forceinline__ const Real* fnormals(const DMesh& m);
-template <> __device__ __forceinline__ const double* fnormals<double>(const DMesh& m) { return m.fnormal; }
-template <> __device__ __forceinline__ const float* fnormals<float>(const DMesh& m) { return m.fnormal32; }
 
 // FieldWeigthing::getFieldVector: VolumeWeighting (VolumeWeightingFW.C:60-67)
 // interpolates cell centre + three triangle points; CellAverage
@@ -132,7 +115,6 @@ __device__ __forceinline__ void field_at(const MoveParams& P, const TetConst& T,
 template <class Real>
 __device__ __forceinline__ void push_boris(const MoveParams& P, const Real* E, const Real* Bv, Real* U, Real tt,
                                       Real zf) {
-    const Real c = Real(kC);
     const Real dt2 = Real(0.5) * tt;
     const Real mU = root_over_c(dot3(U, U));
     const Real g0 = sqrt(Real(1) - mU * mU);
@@ -218,7 +200,6 @@ __device__ __forceinline__ void push_vay(const MoveParams& P, const Real* E, con
 template <class Real>
 __device__ __forceinline__ void push_hc(const MoveParams& P, const Real* E, const Real* Bv, Real* U, Real tt,
                                       Real zf) {
-    const Real c = Real(kC);
     const Real dt2 = Real(0.5) * tt;
     const Real mU = root_over_c(dot3(U, U));
     const Real g0 = sqrt(Real(1) - mU * mU);
