@@ -2014,7 +2014,9 @@ static picgpu_status create_with_mesh(picgpu_ctx* c, const picgpu_config* cfg) {
         }
     }
     CK(cudaMemset(c->st, 0, sizeof(pgd::PcgState)));
-    CK(pgd::pcg_make_plan(int(nc), c->dm.lap_uniform != 0, &c->pcg_plan));
+    // (multigrid contexts never run it)
+    if (cfg->pcg_precond != PICGPU_PRECOND_MULTIGRID || cfg->maxwell_solver != PICGPU_MAXWELL_ELECTROSTATIC)
+        CK(pgd::pcg_make_plan(int(nc), c->dm.lap_uniform != 0, &c->pcg_plan));
     if (c->pcg_plan.fits) {
         const size_t slots = size_t(pgd::pcg_slots(int(nc)));
         if ((s = dalloc(c, &c->pcg_slots, slots))) return s;
