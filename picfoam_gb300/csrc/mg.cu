@@ -44,7 +44,6 @@ constexpr double kEtaMin = 1e-4;   // deepest relative reduction asked of one FP
 // prolongation: 17 and 11 at 48^3, 18 and 10 at 64^3, 20 and 13 at 128^3.
 constexpr float kLinear = 1.25f;
 constexpr long kFuseVoxels = 40000;   // see vcycle()
-constexpr long kSmallVoxels = 600000; // see sum_planes()
 
 // Every kernel of a solve begins with after_previous(): its blocks may be set
 // up while the previous kernel still runs (programmatic dependent launch), and
@@ -77,8 +76,14 @@ struct Interp {
     float w_first[3], w_last[3][3];
 };
 
+// Planes per thread of the kernels that end in a grid-wide sum: each block's
+// ticket costs 1.8 ns at one address (128^3: 25 us per sweep with a sum for 1
+// plane, 14.3 for 4, 13.3 for 8), but the planes' latencies add up.  Microseconds
+// of a solve to 1e-10 with 1, 2, 4 and 8: 48^3 774, 821, 872, 945; 64^3 892, 943,
+// 989, 986; 72^3 1291, 1219, 1232, 1244; 80^3 1438, 1321, 1342, 1460; 88^3 1550,
+// 1449, 1407, 1429; 112^3 2440, 2170, 2043, 2054; 128^3 3245, 2804, 2614, 2571.
 constexpr int kZB = 8;
-int sum_planes(const MgLevel& L) { return L.V <= kSmallVoxels ? 1 : kZB; }
+int sum_planes(const MgLevel& L) { return L.V <= 300000 ? 1 : L.V <= 600000 ? 2 : L.V <= 1700000 ? 4 : kZB; }
 
 Lv view(const MgLevel& L) {
     Lv v{};
@@ -126,11 +131,6 @@ Shape shape(int X, int Y, int Z) {
 
 Shape shape(const MgLevel& L) { return shape(L.n[0], L.n[1], L.n[2]); }
 
-// The level-0 kernels that end in a grid-wide sum give each thread up to kZB
-// z-planes: each block's ticket costs 1.8 ns at one address (128^3: 25 us per
-// sweep with a sum for 1 plane, 14.3 for 4, 13.3 for 8); on small grids one,
-// as the planes' latencies add up (48^3: 6.0 against 6.2 us, with p.q and q.z
-// 5.6 against 6.6).
 Shape shape_sum(const MgLevel& L) {
     Shape s = shape(L);
     s.grid.z = (L.n[2] + sum_planes(L) - 1) / sum_planes(L);
