@@ -73,6 +73,7 @@ struct DMesh {
     const double* bf_normal; // 3 per bface
     const double* bf_area;
     const double* bf_delta;
+    const PatchConst* patches;   // of this mesh: kinds, potentials, areas
     const double* vw_weight; // 8 n_cells
     const int* pi_start;     // n_points + 1
     const int* pi_src;

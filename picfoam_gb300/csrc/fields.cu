@@ -24,7 +24,6 @@
 
 namespace pgd {
 
-__constant__ PatchConst c_patchF;
 
 constexpr double kMu0 = 4.0 * kPi * 1e-7;
 __device__ __forceinline__ double eps0() { return 1.0 / (kMu0 * kC * kC); }
@@ -115,10 +114,11 @@ void launch_corner_E(const DMesh& m, const float* E32, const float* Ept32, float
 }
 
 // FloatingPotential::preUpdate_Boundary (FloatingPotential.C:89-100)
-__global__ void floating_update_kernel(double* qconv, double* sigma, double* grad_bc) {
+__global__ void floating_update_kernel(const PatchConst* __restrict__ pc, double* qconv, double* sigma,
+                                       double* grad_bc) {
     const int p = threadIdx.x;
-    if (p >= c_patchF.n || c_patchF.kind[p] != PICGPU_PATCH_FLOATING) return;
-    sigma[p] += qconv[p] / c_patchF.area[p];
+    if (p >= pc->n || pc->kind[p] != PICGPU_PATCH_FLOATING) return;
+    sigma[p] += qconv[p] / pc->area[p];
     grad_bc[p] = sigma[p] / eps0();
     qconv[p] = 0.0;
 }
@@ -197,9 +197,9 @@ __global__ void rhs_kernel(DMesh m, const double* __restrict__ rho, const double
         const int bf = m.cell_bface[6 * size_t(c) + f];
         if (bf < 0) continue;
         const int pa = m.bf_patch[bf];
-        const int rule = pg::face_rule(c_patchF.kind[pa], c_patchF.phi_bc[pa]);
+        const int rule = pg::face_rule(m.patches->kind[pa], m.patches->phi_bc[pa]);
         if (rule != pg::kRuleNone)
-            t = t + pg::face_rhs(rule, c_patchF.phi[pa], grad_bc[pa], c_patchF.rlc_k[pa], m.bf_area[bf],
+            t = t + pg::face_rhs(rule, m.patches->phi[pa], grad_bc[pa], m.patches->rlc_k[pa], m.bf_area[bf],
                                  m.bf_delta[bf]);
     }
     b[c] = t;
@@ -461,8 +461,8 @@ __device__ __forceinline__ bool boundary_phi(const DMesh& m, const double* grad_
     const int bf = m.cell_bface[6 * size_t(c) + f];
     if (bf < 0) return false;
     const int pa = m.bf_patch[bf];
-    *pf = pg::face_value(pg::face_rule(c_patchF.kind[pa], c_patchF.phi_bc[pa]), c_patchF.phi[pa], grad_bc[pa],
-                         c_patchF.rlc_k[pa], m.bf_delta[bf], phic);
+    *pf = pg::face_value(pg::face_rule(m.patches->kind[pa], m.patches->phi_bc[pa]), m.patches->phi[pa], grad_bc[pa],
+                         m.patches->rlc_k[pa], m.bf_delta[bf], phic);
     return true;
 }
 
@@ -524,8 +524,8 @@ __global__ void boundary_E_kernel(DMesh m, const double* __restrict__ phi,
     const int pa = m.bf_patch[b];
     const double* Ec = E + 3 * size_t(c);
     const double* n = m.bf_normal + 3 * size_t(b);
-    const double sn = pg::face_sn_grad(pg::face_rule(c_patchF.kind[pa], c_patchF.phi_bc[pa]), c_patchF.phi[pa],
-                                       grad_bc[pa], c_patchF.rlc_k[pa], m.bf_delta[b], phi[c]);
+    const double sn = pg::face_sn_grad(pg::face_rule(m.patches->kind[pa], m.patches->phi_bc[pa]), m.patches->phi[pa],
+                                       grad_bc[pa], m.patches->rlc_k[pa], m.bf_delta[b], phi[c]);
     const double En = Ec[0] * n[0] + Ec[1] * n[1] + Ec[2] * n[2];
     if (keep) return;
     for (int a = 0; a < 3; ++a) Eb[3 * size_t(b) + a] = (Ec[a] - En * n[a]) - sn * n[a];
@@ -610,10 +610,6 @@ __global__ void field_energy_kernel(const double* __restrict__ E, const double* 
 // ------------------------------------------------------------ launchers --
 static inline int blocks(long n, int bs) { return int((n + bs - 1) / bs); }
 
-cudaError_t fields_set_patches(const PatchConst& p) {
-    return cudaMemcpyToSymbol(c_patchF, &p, sizeof p);
-}
-
 void launch_charge_update(const DMesh& m, int vw, int fixed, double fix_scale, const double* ccd,
                           const double* vtxd, const long long* ccf, const long long* vtxf,
                           double space_charge, double* rho, cudaStream_t s) {
@@ -621,8 +617,8 @@ void launch_charge_update(const DMesh& m, int vw, int fixed, double fix_scale, c
                                                                 vtxf, space_charge, rho);
 }
 
-void launch_floating_update(double* qconv, double* sigma, double* grad_bc, cudaStream_t s) {
-    floating_update_kernel<<<1, 32, 0, s>>>(qconv, sigma, grad_bc);
+void launch_floating_update(const DMesh& m, double* qconv, double* sigma, double* grad_bc, cudaStream_t s) {
+    floating_update_kernel<<<1, 32, 0, s>>>(m.patches, qconv, sigma, grad_bc);
 }
 
 void launch_circuit_pre(const CircuitParams& P, double src, double* qconv, double* grad_bc, pg::CircuitState* S,

@@ -61,7 +61,6 @@ struct SpeciesValues {
     double v[PICGPU_MAX_SPECIES];
 };
 
-cudaError_t fields_set_patches(const PatchConst& p);
 void launch_charge_update_mixed(const DMesh& m, int vw, const SpeciesValues& sv, const unsigned long long* acc9,
                                 double* vtx, double space_charge, double* rho, cudaStream_t s);
 void launch_corner_E(const DMesh& m, const float* E32, const float* Ept32, float4* Ec4, cudaStream_t s);
@@ -69,7 +68,7 @@ int pcg_blocks(int n);
 void launch_charge_update(const DMesh& m, int vw, int fixed, double fix_scale, const double* ccd,
                           const double* vtxd, const long long* ccf, const long long* vtxf,
                           double space_charge, double* rho, cudaStream_t s);
-void launch_floating_update(double* qconv, double* sigma, double* grad_bc, cudaStream_t s);
+void launch_floating_update(const DMesh& m, double* qconv, double* sigma, double* grad_bc, cudaStream_t s);
 
 // Circuit model of a context (constant over a run).
 struct CircuitParams {

@@ -5,7 +5,7 @@
 
 namespace pgd {
 
-cudaError_t move_fp64_set_tables(const TetConst& t, const PatchConst& p);
+cudaError_t move_fp64_set_tables(const TetConst& t);
 void launch_move_fp64(const MoveParams& P, int sms, cudaStream_t s);
 // Blocks per SM of the FP32 mover outside of graphs: 5, which are resident, or
 // three rounds of them.  The chunks differ in the faces that their parcels

@@ -1230,7 +1230,7 @@ picgpu_status one_step(picgpu_ctx* c, picgpu_step_stats* stats, bool fields) {
         if ((s = charge_update(c))) return s;
     }
     if (!fields) return PICGPU_OK;
-    pgd::launch_floating_update(c->qconv, c->sigma, c->grad_bc, c->stream);
+    pgd::launch_floating_update(c->dm, c->qconv, c->sigma, c->grad_bc, c->stream);
     c->launches++;
     // circuit models around the field solve (PICCloud.C:1457-1464); the
     // source and the averaging factor are evaluated here, on the host
@@ -1826,7 +1826,7 @@ static picgpu_status create_with_mesh(picgpu_ctx* c, const picgpu_config* cfg) {
         P.dt = cfg->dt;
         if (cc.model == PICGPU_CIRCUIT_RLC) c->pc.rlc_k[cc.cathode_patch] = rc.k;
     }
-    CK(pgd::move_fp64_set_tables(c->tc, c->pc));
+    CK(pgd::move_fp64_set_tables(c->tc));
     CK(pgd::init_set_tables(c->tc));
     {
         std::vector<double> tv(12 * size_t(std::max(m.n_classes, 1)), 0.0);
@@ -1870,7 +1870,6 @@ static picgpu_status create_with_mesh(picgpu_ctx* c, const picgpu_config* cfg) {
         if ((us = dalloc(c, &c->xq_count, size_t(c->xq_cap))) || (us = dalloc(c, &c->xq_start, size_t(c->xq_cap))))
             return us;
     }
-    CK(pgd::fields_set_patches(c->pc));
     CK(pgd::collide_set_tables(c->tc));
 
     // mesh arrays
@@ -1911,6 +1910,8 @@ static picgpu_status create_with_mesh(picgpu_ctx* c, const picgpu_config* cfg) {
         if ((s = upload(c, &ptr_, vec))) return s;     \
         d.field = ptr_;                                \
     }
+    const std::vector<pgd::PatchConst> patch_table{c->pc};
+    UP(patches, patch_table, pgd::PatchConst);
     UP(cell_class, m.cell_class, int);
     UP(nbr, m.nbr, int);
     UP(cell_pt, m.cell_pt, int);
@@ -2921,7 +2922,7 @@ picgpu_status picgpu_set_field(picgpu_ctx* c, int which, const double* in, size_
             if (c->m.patches[p].p.kind == PICGPU_PATCH_FLOATING) sg[p] = in[p];
         CK(cudaMemcpy(c->sigma, sg.data(), np * sizeof(double), cudaMemcpyHostToDevice));
         // the floating update with an empty accumulator: gradient sigma / eps0
-        pgd::launch_floating_update(c->qconv, c->sigma, c->grad_bc, c->stream);
+        pgd::launch_floating_update(c->dm, c->qconv, c->sigma, c->grad_bc, c->stream);
         c->launches++;
         CK(cudaStreamSynchronize(c->stream));
         return PICGPU_OK;

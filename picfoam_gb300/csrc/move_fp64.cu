@@ -9,7 +9,6 @@
 namespace pgd {
 
 __constant__ TetConst c_tet64;
-__constant__ PatchConst c_patch64;
 
 // An FP64 warp instruction holds its quarter of an SM for 64 cycles whether one
 // lane needs it or all, so the mover is bound by the number of FP64 warp
@@ -124,7 +123,7 @@ __device__ __forceinline__ void sync_velocity(const MoveParams& P, const TetCons
 // of the hit.
 __device__ __forceinline__ bool hit_patch(const MoveParams& P, const TetConst& T, PState<double>& s, int patch,
                                           double sf, unsigned* walls, bool* resync) {
-    const int kind = c_patch64.kind[patch];
+    const int kind = P.m.patches->kind[patch];
     if (kind == PICGPU_PATCH_ABSORB) return false;
     // FloatingPotential deletes every parcel; a circuit electrode
     // (circuitRLC.C:268-288) deletes charged parcels and reflects neutral ones
@@ -408,11 +407,7 @@ void launch_push_only(const MoveParams& P, bool fp32, double tt, int grid, cudaS
     else push_only_kernel<double><<<grid, 256, 0, s>>>(P, tt);
 }
 
-cudaError_t move_fp64_set_tables(const TetConst& t, const PatchConst& p) {
-    cudaError_t e = cudaMemcpyToSymbol(c_tet64, &t, sizeof t);
-    if (e != cudaSuccess) return e;
-    return cudaMemcpyToSymbol(c_patch64, &p, sizeof p);
-}
+cudaError_t move_fp64_set_tables(const TetConst& t) { return cudaMemcpyToSymbol(c_tet64, &t, sizeof t); }
 
 void launch_move_fp64(const MoveParams& P, int sms, cudaStream_t s) {
     // as many warps as the chip holds, each with an equal share of the rows of
