@@ -5,8 +5,9 @@
 // full voxel grid (voxels of removed box cells are holes: no equation, value
 // zero), so every level addresses its neighbours by index arithmetic.  Level
 // l + 1 aggregates 2x2x2 voxels of level l (ceil(n/2) aggregates per axis);
-// its operator is the Galerkin product P^T A P with piecewise-constant P (the
-// correction itself is prolonged linearly):
+// its operator is the Galerkin product P^T A P with piecewise-constant P, but
+// that an aggregate which is not full counts its coupling to given potentials
+// twice (the correction itself is prolonged linearly):
 // face couplings summed across aggregate faces, diagonals and internal
 // couplings summed into the diagonal.  One preconditioner application is a
 // V-cycle: weighted-Jacobi sweeps before and after the scaled coarse

@@ -49,7 +49,7 @@
 // the sums of the chunks.
 // Per iteration on GB300 (before: with arrival counters throughout, and as the
 // two-kernel iteration of fields.cu in a CUDA graph): 5917 cells 4.2 us (6.4,
-// 18.6), 27,000 cells 5.5 (7.2, 19), 64,000 cells 6.9 (8.1), 91,125 cells 9.0
+// 18.6; 4.0 with its end in leave()), 27,000 cells 5.5 (7.2, 19), 64,000 cells 6.9 (8.1), 91,125 cells 9.0
 // (9.3, 19.5; 10.0 with slots), 262,144 cells 15.8 (15.7, 21; 18.4 with slots
 // for u), 512,000 cells 25.3 (27.4); one block of 128 cells 2 us (2, 11.5).
 #include "fields.h"

@@ -175,7 +175,7 @@ __global__ void pool_kernel(ConvGrid g, int C, const __nv_bfloat16* __restrict__
 
 // h = bf16(g * (a > 0)), g FP32 [n], a BF16 [n]; eight values per thread (n is a
 // multiple of the channels, 8 at least), 16-byte loads and stores: one value
-// per thread took 74 us of a 64 x 64 x 32 network's gradient.
+// per thread took 74 us of a 64 x 64 x 64 network's gradient.
 __global__ void relu_mask_kernel(long n, const float* __restrict__ gr, const __nv_bfloat16* __restrict__ a,
                                  __nv_bfloat16* __restrict__ h) {
     const long i = 8 * (long(blockIdx.x) * blockDim.x + threadIdx.x);
@@ -196,7 +196,7 @@ __global__ void relu_mask_kernel(long n, const float* __restrict__ gr, const __n
 // children of g_cat[child][c].
 // One thread per value, the channels of a voxel together: a thread per coarse
 // voxel, with 16 blocks on the smaller of two grids and neighbours a voxel's
-// channels apart, took 297 us of the 2255 of a 64 x 64 x 32 network's gradient
+// channels apart, took 297 us of the 2255 of a 64 x 64 x 64 network's gradient
 // (1990 now; 1926 with the masks and pooling below in wide accesses).
 template <int C1, int C2>
 __global__ void split_cat_kernel(ConvGrid g, const float* __restrict__ gcat, float* __restrict__ gskip,
